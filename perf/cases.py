@@ -74,8 +74,9 @@ def _log(rng, lo, hi):
 def draw(rng):
     kind = rng.choice(["unwrap", "lscm", "lscm", "arap", "arap", "validate", "energy", "energy", "report", "pack"])
     if kind in ("unwrap", "lscm", "arap"):
-        case = {"kind": kind, "islands": _log(rng, 1, 1200), "tmin": _log(rng, 20, 200),
-                "tmax": _log(rng, 400, 24000)}
+        n = _log(rng, 1, 1200)
+        case = {"kind": kind, "islands": n, "tmin": _log(rng, 20, 200) if n >= 16 else _log(rng, 300, 600),
+                "tmax": _log(rng, 700, 24000)}
         if kind != "lscm":
             case["iters"] = rng.randint(4, 20)
         if kind == "arap" and rng.random() < 0.25:
@@ -86,7 +87,7 @@ def draw(rng):
                 "atlas": rng.choice([1024, 2048, 4096]), "padding": rng.choice([2, 4]),
                 "preserve": rng.random() < 0.5}
     if kind == "energy":
-        return {"kind": kind, "islands": _log(rng, 1, 400), "tmin": _log(rng, 100, 1000),
+        return {"kind": kind, "islands": _log(rng, 1, 400), "tmin": _log(rng, 300, 1000),
                 "tmax": _log(rng, 2000, 60000), "energy": rng.randint(0, 1), "grad_positions": rng.random() < 0.5}
     if kind == "report":
         return {"kind": kind, "islands": _log(rng, 1, 500), "tmin": _log(rng, 20, 200),
