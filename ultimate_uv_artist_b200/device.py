@@ -277,7 +277,8 @@ class DevicePlan:
             D.sizes, D.scratch, D.scratch_bytes = sizes.data_ptr(), scratch.data_ptr(), int(nb.value)
             s = stream if stream is not None else torch.cuda.current_stream(d)
             check(L.uva_dplan_build(C.byref(D), C.c_void_p(s.cuda_stream)), "uva_dplan_build")
-        self._pending = (D, sizes, dev, s, d, Td, scratch, T32)
+        # the descriptor's arrays stay alive until the slot pass has read them
+        self._pending = (D, sizes, dev, s, d, (vd, td, Td), scratch, T32)
         self.dev_arrays = None
         if finish:
             self.finish()
