@@ -225,11 +225,19 @@ typedef struct uva_batch {
                                                 /* rc: t*3*2 corner RHS terms */
     float*  r32;  float*  d32;  float*  p32;  float* q32;
     uva_island_status* status;                  /* nc                         */
-    int32_t* work;            /* >= 4 ints, zeroed by the callee per launch     */
+    int32_t* work;            /* >= 4 ints (8 with direct), zeroed per launch   */
     float*  hist;             /* 16*n floats (optional): the last 4 ARAP updates
                                  and their images under the operator, FP32 by
                                  solver row, for the start of each global step;
                                  null: 2 updates kept in p32/d32/q32/r32        */
+    /* direct solver of islands up to 16,384 vertices (all optional; null: CG) */
+    int32_t* band;            /* n + n/16 + 5*nc ints: elimination order, skyline
+                                 and state per island, written by the setup     */
+    unsigned char* direct;    /* factor scratch of uva_lscm / uva_arap           */
+    const int64_t* direct_ofs;/* device, 2*(direct_slots+1): byte offsets of the
+                                 CTAs' parts, for ARAP then for LSCM: part j is
+                                 sized for the j-th island of `order`            */
+    int32_t direct_slots;     /* CTAs of the direct launches                     */
 } uva_batch;
 
 /* Island size classes of one persistent launch (see uva_arap): islands are

@@ -30,6 +30,7 @@ ST_BADCLASS = 16
 PLAN_NSIZES = 9
 STEP_SETUP, STEP_LSCM, STEP_ARAP = 1, 2, 4
 CLASS_BIG, CLASS_MID, CLASS_SMALL = 8192, 2048, 256
+DIRECT_MAX_N = 16384   # islands above keep the CG path (direct.cuh)
 (PLAN_NC, PLAN_N, PLAN_T, PLAN_E, PLAN_NSLICES, PLAN_NSLOTS, PLAN_NBVERTS, PLAN_MAXROWS, PLAN_NCOARSE) = range(9)
 
 vp = C.c_void_p
@@ -55,7 +56,8 @@ class BatchDesc(C.Structure):
                 ("P", vp), ("frame", vp), ("wtri", vp), ("tscale", vp), ("wedge", vp), ("slot_cw", vp),
                 ("wdiag", vp), ("dinv", vp), ("pins", vp), ("wpin", vp), ("U", vp),
                 ("x64", vp), ("b64", vp), ("rc", vp), ("r32", vp), ("d32", vp), ("p32", vp), ("q32", vp),
-                ("status", vp), ("work", vp), ("hist", vp)]
+                ("status", vp), ("work", vp), ("hist", vp),
+                ("band", vp), ("direct", vp), ("direct_ofs", vp), ("direct_slots", i32)]
 
 
 class DPlanDesc(C.Structure):

@@ -28,6 +28,8 @@
 #include <vector>
 
 #include "common.cuh"
+#include "direct.cuh"
+#include "island.cuh"
 
 using namespace uva;
 
@@ -533,11 +535,6 @@ __device__ __forceinline__ Isl load_island(const uva_batch& b, int isl) {
 }
 
 __device__ __forceinline__ int agg_of(const Isl& I, int i) { return I.aggsh >= 0 ? (i >> I.aggsh) : i / I.agg; }
-
-// Packed slot column: island row in the low 24 bits, twice the LSCM
-// boundary coupling (a small integer) in the high 8 bits.
-__device__ __forceinline__ int slot_row(int x) { return x & 0xFFFFFF; }
-__device__ __forceinline__ float slot_c2(int x) { return static_cast<float>(x >> 24); }
 
 __device__ __forceinline__ void row_slots(const uva_batch&, const Isl& I, int i, int& q0, int& width) {
     const int s = i >> 5;
@@ -1246,118 +1243,6 @@ __device__ __forceinline__ int refine_solve(const uva_batch& b, const Isl& I, co
     return total;
 }
 
-// ---- local step (per triangle): closest rotation + corner RHS terms.
-// BATCH: engine/gpu.py:165-182. PARAM: engine/param.py:206-233, 457-474.
-__device__ __forceinline__ void local_terms(const uva_batch& b, const Isl& I, int f, const double2* U, bool batch,
-                                            double& energy, int& flip) {
-    const int4 tv = reinterpret_cast<const int4*>(b.tri4)[f];
-    const double4 fr = reinterpret_cast<const double4*>(b.frame)[f];
-    const double4 wt = reinterpret_cast<const double4*>(b.wtri)[f];
-    const double2 u0 = U[I.v0 + tv.x], u1 = U[I.v0 + tv.y], u2 = U[I.v0 + tv.z];
-    const double x1 = fr.x, x2 = fr.y, y2 = fr.z;
-    const double du1x = u1.x - u0.x, du1y = u1.y - u0.y, du2x = u2.x - u0.x, du2y = u2.y - u0.y;
-    double c = 1.0, s = 0.0;
-    const double sar = du1x * du2y - du2x * du1y;
-    flip = sar <= 0.0 ? 1 : 0;
-    energy = 0.0;
-    if (batch) {
-        if (wt.w != 0.0) {
-            const double j00 = du1x / x1, j10 = du1y / x1;
-            const double j01 = (du2x - j00 * x2) / y2, j11 = (du2y - j10 * x2) / y2;
-            const double ca = j00 + j11, cb = j10 - j01;
-            if (isfinite(ca) && isfinite(cb)) {
-                const double h = hypot(ca, cb);
-                if (h > 0.0) { c = ca / h; s = cb / h; }
-            } else if (!isnan(ca) && !isnan(cb)) {
-                const double th = atan2(cb, ca);
-                c = cos(th); s = sin(th);
-            }
-        }
-        const double sc = static_cast<double>(b.tscale[f]);
-        c *= sc; s *= sc;
-    } else if (fabs(x1 * y2) >= 1e-300) {
-        const double j00 = du1x / x1, j10 = du1y / x1;
-        const double j01 = (du2x - j00 * x2) / y2, j11 = (du2y - j10 * x2) / y2;
-        double ca = j00 + j11, cb = j10 - j01;
-        double h = sqrt(ca * ca + cb * cb);
-        if (h < 1e-300) { ca = 1.0; cb = 0.0; h = 1.0; }
-        c = ca / h; s = cb / h;
-        const double qe = 0.5 * (j00 + j11), qh = 0.5 * (j10 - j01);
-        const double rf = 0.5 * (j00 - j11), rg = 0.5 * (j10 + j01);
-        const double q = sqrt(qe * qe + qh * qh), r = sqrt(rf * rf + rg * rg);
-        energy = fr.w * ((q + r - 1.0) * (q + r - 1.0) + (q - r - 1.0) * (q - r - 1.0));
-    }
-    // edge k runs corner k+1 -> k+2; frame corners (0,0), (x1,0), (x2,y2)
-    const double cxs[3] = {0.0, x1, x2}, cys[3] = {0.0, 0.0, y2};
-    const double wk[3] = {wt.x, wt.y, wt.z};
-    double vx[3], vy[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int i = (k + 1) % 3, j = (k + 2) % 3;
-        const double dx = cxs[i] - cxs[j], dy = cys[i] - cys[j];
-        vx[k] = wk[k] * (c * dx - s * dy);
-        vy[k] = wk[k] * (s * dx + c * dy);
-    }
-    double2* rc = reinterpret_cast<double2*>(b.rc);
-#pragma unroll
-    for (int cc = 0; cc < 3; ++cc) {
-        const int kp = (cc + 2) % 3, km = (cc + 1) % 3;
-        rc[3 * f + cc] = make_double2(vx[kp] - vx[km], vy[kp] - vy[km]);
-    }
-}
-
-// Flip-safe step bound of one triangle (smallest positive root of the
-// signed-area quadratic). BATCH: gpu.py:204-227, PARAM: param.py:259-291.
-__device__ __forceinline__ double step_bound(const uva_batch& b, const Isl& I, int f, const double2* U, const double2* X,
-                                             bool batch) {
-    const int4 tv = reinterpret_cast<const int4*>(b.tri4)[f];
-    const double2 u0 = U[I.v0 + tv.x], u1 = U[I.v0 + tv.y], u2 = U[I.v0 + tv.z];
-    const int* vr = b.vert_row + I.v0;
-    const double2 x0 = X[I.v0 + vr[tv.x]], x1 = X[I.v0 + vr[tv.y]], x2 = X[I.v0 + vr[tv.z]];
-    const double2 d0 = make_double2(x0.x - u0.x, x0.y - u0.y), d1 = make_double2(x1.x - u1.x, x1.y - u1.y),
-                  d2 = make_double2(x2.x - u2.x, x2.y - u2.y);
-    const double ux1 = u1.x - u0.x, uy1 = u1.y - u0.y, ux2 = u2.x - u0.x, uy2 = u2.y - u0.y;
-    const double dx1 = d1.x - d0.x, dy1 = d1.y - d0.y, dx2 = d2.x - d0.x, dy2 = d2.y - d0.y;
-    const double C = ux1 * uy2 - ux2 * uy1;
-    const double B = ux1 * dy2 + dx1 * uy2 - ux2 * dy1 - dx2 * uy1;
-    const double A = dx1 * dy2 - dx2 * dy1;
-    const double big = 1e30;
-    if (!(C > 0.0)) return big;
-    if (batch) {
-        double t = big;
-        if (fabs(A) < 1e-30) {
-            if (B < 0.0) t = -C / B;
-        } else {
-            const double disc = B * B - 4.0 * A * C;
-            if (disc >= 0.0) {
-                const double sq = sqrt(disc);
-                const double r1 = (-B - sq) / (2.0 * A), r2 = (-B + sq) / (2.0 * A);
-                if (r1 > 0.0) t = fmin(t, r1);
-                if (r2 > 0.0) t = fmin(t, r2);
-            }
-        }
-        return isnan(t) ? big : t;
-    }
-    if (A == 0.0 || fabs(A) < 1e-30 * fmax(fabs(B), 1e-300)) return B < 0.0 ? -C / B : big;
-    const double disc = B * B - 4.0 * A * C;
-    if (disc < 0.0) return big;
-    const double sq = sqrt(disc);
-    const double r1 = (-B - sq) / (2.0 * A), r2 = (-B + sq) / (2.0 * A);
-    double t = big;
-    if (r1 > 0.0 && r1 < t) t = r1;
-    if (r2 > 0.0 && r2 < t) t = r2;
-    return t;
-}
-
-// 1 if triangle f is folded at U: negative signed UV area with a valid frame
-// (engine/hier.py:549)
-__device__ __forceinline__ int folded_tri(const uva_batch& b, const Isl& I, int f, const double2* U) {
-    if (reinterpret_cast<const double4*>(b.wtri)[f].w == 0.0) return 0;
-    const int4 tv = reinterpret_cast<const int4*>(b.tri4)[f];
-    const double2 a = U[I.v0 + tv.x], c1 = U[I.v0 + tv.y], c2 = U[I.v0 + tv.z];
-    return ((c1.x - a.x) * (c2.y - a.y) - (c2.x - a.x) * (c1.y - a.y)) < 0.0 ? 1 : 0;
-}
-
 // ---- ARAP outer iterations of one island (gpu.py:230-249 / param.py:379-414)
 template <int NTT, int R>
 __device__ __forceinline__ void solve_arap(const uva_batch& b, const uva_solve_params& prm, Team<NTT>& tm, const Isl& I) {
@@ -1391,7 +1276,7 @@ __device__ __forceinline__ void solve_arap(const uva_batch& b, const uva_solve_p
         double ev[2] = {0.0, 0.0};
         for (int f = I.f0 + tid; f < I.f0 + I.nt; f += NTT) {
             double e; int fl;
-            local_terms(b, I, f, U, batch, e, fl);
+            local_terms(b, I.v0, f, U, batch, e, fl);
             ev[0] += e; ev[1] += fl;
         }
         if (!batch) {
@@ -1452,8 +1337,8 @@ __device__ __forceinline__ void solve_arap(const uva_batch& b, const uva_solve_p
             double tmin = 1e30;
             int folded = 0;
             for (int f = I.f0 + tid; f < I.f0 + I.nt; f += NTT) {
-                tmin = fmin(tmin, step_bound(b, I, f, U, x64, batch));
-                if (prm.fold_step) folded |= folded_tri(b, I, f, U);
+                tmin = fmin(tmin, step_bound(b, I.v0, f, U, x64, batch));
+                if (prm.fold_step) folded |= folded_tri(b, I.v0, f, U);
             }
             tmin = team_min(tm, tmin);
             if (prm.fold_step) folded = team_or(tm, folded);   // folded islands: plain ARAP step
@@ -1580,18 +1465,6 @@ __device__ __forceinline__ void solve_lscm(const uva_batch& b, const uva_solve_p
     tm.sync();
 }
 
-__device__ __forceinline__ long long global_ns() {
-    long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ unsigned sm_id() {
-    unsigned r;
-    asm("mov.u32 %0, %%smid;" : "=r"(r));
-    return r;
-}
-
 // A class-G island that the class-W team solves: above kWideMin vertices,
 // and its coarse g and y fit the batch's cpart after the team's header.
 // (Its reduction partials and warp sums fit its own block of the batch's
@@ -1620,6 +1493,7 @@ __device__ __forceinline__ void run_class(const uva_batch& b, const uva_solve_pa
         }
         if (lo + qi >= hi) break;
         Isl I = load_island<OP>(b, b.order[lo + qi]);
+        if (b.direct && band_info(b, I.id)[3]) continue;   // solved by the direct path
         if (R == 0 && skip_wide && wide_island(b, I)) continue;   // solved by k_wide
         if (R > 0 && I.n > NTT * R) {   // the team's shared-memory vectors hold NTT * R rows
             if (tm.tid == 0) {
@@ -1707,6 +1581,7 @@ __global__ void __launch_bounds__(KB, 1) k_islands(uva_batch b, uva_solve_params
     __shared__ __align__(16) float coarse_buf[1024];   // g and y of the coarse level (CTA: 512 each; sub-team: 128 each)
     __shared__ int sc_buf[288];          // slice pointers (CTA: 288; sub-team: 72 each; warp: 9 each)
     __shared__ __nv_bfloat16 dinv_buf[KB * RB];   // Jacobi (CTA: 8192; sub-team: 2048; warp: 256)
+    if (b.direct && b.work[kWorkLeft] == 0) return;   // the direct path solved every island
     const bool rev = static_cast<int>(blockIdx.x) < nrev;
     auto whole_cta = [&]() {
         Team<KB> tm{static_cast<int>(threadIdx.x), 0, 0, redd, redf, redi, &slots[0], nullptr, nullptr, nullptr,
@@ -2056,6 +1931,12 @@ bool check_classes(const uva_batch* b) {
     return true;
 }
 
+// ARAP calls of fewer iterations keep the CG path: the factor is paid for
+// once per call.
+constexpr int kDirectMinIters = 3;
+
+bool direct_ready(const uva_batch* b) { return b->band && b->direct && b->direct_ofs && b->direct_slots > 0; }
+
 template <Op OP>
 int launch_islands(const uva_batch* b, const uva_solve_params* prm, cudaStream_t s) {
     if (!check_classes(b)) {
@@ -2064,8 +1945,12 @@ int launch_islands(const uva_batch* b, const uva_solve_params* prm, cudaStream_t
     }
     cudaError_t e = ensure_islands_attr<OP>();
     if (e != cudaSuccess) return uva_cuda_status(e, "uva_islands/cudaFuncSetAttribute");
-    e = cudaMemsetAsync(b->work, 0, sizeof(int32_t) * 4, s);
+    e = cudaMemsetAsync(b->work, 0, sizeof(int32_t) * (b->direct ? 8 : 4), s);
     if (e != cudaSuccess) return uva_cuda_status(e, "uva_islands/memset");
+    if (b->direct) {   // the islands it leaves (info[3] == 0) are solved below
+        const int rc = uva_direct_launch(b, prm, OP == OP_LSCM, s);
+        if (rc != UVA_OK) return rc;
+    }
     const int big = b->class_ofs[2];                        // islands that take a whole CTA
     const int small = b->class_ofs[4] - b->class_ofs[2];    // islands for sub-teams / warps
     const int want = big + (small + 3) / 4;
@@ -2398,6 +2283,10 @@ extern "C" int uva_batch_setup(uva_batch* b, void* stream) {
     UVA_CHECK_LAUNCH("uva_batch_setup/rows");
     k_far_pair<<<(b->nc + 127) / 128, 128, 0, s>>>(*b);
     UVA_CHECK_LAUNCH("uva_batch_setup/pins");
+    if (b->band) {
+        const int rc = uva_direct_order(b, s);
+        if (rc != UVA_OK) return rc;
+    }
     if (b->coarse_a && b->coarse_l && b->coarse_work) {
         const cudaError_t e = ensure_coarse_attr();   // 128 KB of dynamic shared memory
         if (e != cudaSuccess) return uva_cuda_status(e, "uva_batch_setup/coarse attribute");
@@ -2414,7 +2303,9 @@ extern "C" int uva_batch_setup(uva_batch* b, void* stream) {
 extern "C" int uva_arap(uva_batch* b, const uva_solve_params* prm, void* stream) {
     if (!check_batch(b) || !prm) { uva_set_error("uva_arap: bad arguments"); return UVA_E_ARG; }
     if (b->nc == 0 || prm->iters <= 0) return UVA_OK;
-    return launch_islands<OP_ARAP>(b, prm, static_cast<cudaStream_t>(stream));
+    uva_batch w = *b;
+    if (prm->iters < kDirectMinIters || !direct_ready(b)) w.direct = nullptr;
+    return launch_islands<OP_ARAP>(&w, prm, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int uva_slim_scratch_bytes(const uva_batch* b, int64_t* bytes) {
@@ -2439,7 +2330,9 @@ extern "C" int uva_slim(uva_batch* b, const uva_solve_params* prm, double* scrat
 extern "C" int uva_lscm(uva_batch* b, const uva_solve_params* prm, void* stream) {
     if (!check_batch(b) || !prm) { uva_set_error("uva_lscm: bad arguments"); return UVA_E_ARG; }
     if (b->nc == 0) return UVA_OK;
-    return launch_islands<OP_LSCM>(b, prm, static_cast<cudaStream_t>(stream));
+    uva_batch w = *b;
+    if (!direct_ready(b)) w.direct = nullptr;
+    return launch_islands<OP_LSCM>(&w, prm, static_cast<cudaStream_t>(stream));
 }
 
 // ------------------------------------------------------------------ step graphs
@@ -2463,6 +2356,7 @@ extern "C" int uva_step_graph_create(uva_batch* b, int32_t parts, const uva_solv
     cudaError_t e = ensure_islands_attr<OP_ARAP>();
     if (e == cudaSuccess) e = ensure_islands_attr<OP_LSCM>();
     if (e == cudaSuccess) e = ensure_coarse_attr();
+    if (e == cudaSuccess) e = uva_direct_attributes();
     if (e != cudaSuccess) return uva_cuda_status(e, "uva_step_graph_create/attributes");
     sm_count();
     cudaStream_t cs = nullptr;
@@ -2572,6 +2466,7 @@ extern "C" int uva_arap_noalloc(const uva_batch* b, const uva_solve_params* prm,
     const int rc = noalloc_scratch(&base);
     if (rc != UVA_OK) return rc;
     uva_batch w = *b;
+    w.direct = nullptr;   // the caller's scratch too
     size_t off = 0;
     w.work = reinterpret_cast<int32_t*>(base + off); off += kNaWork;
     w.x64 = reinterpret_cast<double*>(base + off); off += kNaX64;

@@ -441,6 +441,26 @@ def concat_charts(charts, with_uv=True, with_t=True):
     return P, T, U, ca.vofs, ca.tofs
 
 
+def direct_parts(nv, slots):
+    """Byte offsets (2, slots + 1) of the direct solver's scratch, ARAP then
+    LSCM: one part per CTA, sized for the CTA's first island (islands of
+    ``nv`` vertices are taken largest first, so the later ones are smaller).
+    A planar chart's factor has about 0.95 sqrt(n) columns per row in
+    breadth-first order; the part holds 1.45 sqrt(n) and two blocks of 16
+    (at most 16 blocks), a ring of 256 blocks, and the solve's vectors. An
+    island whose factor needs more keeps the CG path."""
+    n = np.sort(np.asarray(nv, np.int64))[::-1][:slots].astype(np.float64)
+    n = np.where(n > _lib.DIRECT_MAX_N, 0, n)
+    nblk = np.ceil(n / 16)
+    blocks = nblk * np.minimum(np.ceil(1.45 * np.sqrt(n) / 16 + 2), 16) + 256
+    ofs = np.zeros((2, slots + 1), np.int64)
+    for k, (block, vecs) in enumerate(((2048, 3), (4096, 1))):
+        part = np.where(n > 0, blocks * block + 256 * nblk * vecs, 0).astype(np.int64)
+        ofs[k, 1:len(n) + 1] = np.cumsum((part + 255) // 256 * 256)
+        ofs[k, len(n) + 1:] = ofs[k, len(n)]
+    return ofs
+
+
 class DeviceBatch:
     """Islands resident on one CUDA device, ready for the uva_* kernels."""
 
@@ -531,6 +551,12 @@ class DeviceBatch:
             self.status = torch.zeros((nc, C.sizeof(_lib.IslandStatus)), dtype=torch.uint8, device=d)
             self.work = torch.zeros(8, dtype=torch.int32, device=d)
             self.rev_ctas = tuned["rev_ctas"] if tuned is not None else 0   # schedule knob (autotune.tune)
+            # direct solver: elimination order (written by the setup) and the
+            # parts of the factor scratch, which every call allocates
+            self.band = torch.empty(self.n + self.n // 16 + 5 * nc + 1, dtype=torch.int32, device=d)
+            self.direct_slots = min(nc, 2 * torch.cuda.get_device_properties(d).multi_processor_count)
+            self._direct_parts = direct_parts(np.diff(plan.vofs.astype(np.int64)), self.direct_slots)
+            self.direct_ofs = up(self._direct_parts)
         self.desc = self._make_desc()
         self.setup()
 
@@ -546,9 +572,26 @@ class DeviceBatch:
                      "vt_ptr", "vt", "vflags", "bofs", "bverts", "order", "row_vert", "vert_row", "agg_rows", "cofs",
                      "coarse_a", "coarse_l", "coarse_work", "cpart", "P", "frame", "wtri", "tscale", "wedge",
                      "slot_cw", "wdiag", "dinv", "pins", "wpin", "U", "x64", "b64", "rc", "r32", "d32", "p32",
-                     "q32", "status", "work", "hist"):
+                     "q32", "status", "work", "hist", "band", "direct_ofs"):
             setattr(D, name, getattr(self, name).data_ptr())
+        D.direct_slots = self.direct_slots
         return D
+
+    def _with_direct(self, *kinds):
+        """(descriptor, scratch): the batch's descriptor with factor scratch
+        for the calls of ``kinds``, from torch's caching allocator on the
+        batch's stream; without memory for it the descriptor as it is (CG)."""
+        nbytes = max(int(self._direct_parts[0 if k == "arap" else 1][-1]) for k in kinds)
+        if nbytes == 0:
+            return self.desc, None
+        try:
+            with (torch.cuda.stream(self.stream) if self.stream is not None else contextlib.nullcontext()):
+                scratch = torch.empty(nbytes, dtype=torch.uint8, device=self.dev)
+        except torch.cuda.OutOfMemoryError:
+            return self.desc, None
+        D = _lib.BatchDesc.from_buffer_copy(self.desc)
+        D.direct = scratch.data_ptr()
+        return D, scratch
 
     def _refresh_u(self):
         """Re-point the descriptor after U was replaced by a new tensor."""
@@ -578,12 +621,14 @@ class DeviceBatch:
     def lscm(self, **kw):
         kw.setdefault("rev_ctas", self.rev_ctas)
         prm = self.params("lscm", **kw)
-        check(_lib.lib().uva_lscm(C.byref(self.desc), C.byref(prm), self._stream()), "uva_lscm")
+        D, scratch = self._with_direct("lscm")
+        check(_lib.lib().uva_lscm(C.byref(D), C.byref(prm), self._stream()), "uva_lscm")
 
     def arap(self, iters=8, line_search=True, energy_tol=0.0, **kw):
         kw.setdefault("rev_ctas", self.rev_ctas)
         prm = self.params("arap", iters=iters, line_search=line_search, energy_tol=energy_tol, **kw)
-        check(_lib.lib().uva_arap(C.byref(self.desc), C.byref(prm), self._stream()), "uva_arap")
+        D, scratch = self._with_direct("arap") if prm.iters > 0 else (self.desc, None)
+        check(_lib.lib().uva_arap(C.byref(D), C.byref(prm), self._stream()), "uva_arap")
 
     def slim(self, iters=10, energy_tol=1e-5, cg_tol=1e-13, cg_max=50000):
         """SLIM iterations of every island (uva_slim; PARAM semantics)."""
@@ -713,7 +758,9 @@ class StepGraph:
         self._lp = db.params("lscm", **lscm_kw)
         self._ap = db.params("arap", iters=max(arap_iters, 1), line_search=line_search, **arap_kw)
         h = C.c_void_p()
-        check(_lib.lib().uva_step_graph_create(C.byref(db.desc), parts, C.byref(self._lp), C.byref(self._ap),
+        kinds = (["lscm"] if lscm else []) + (["arap"] if arap_iters > 0 else [])
+        D, self._scratch = db._with_direct(*kinds) if kinds else (db.desc, None)
+        check(_lib.lib().uva_step_graph_create(C.byref(D), parts, C.byref(self._lp), C.byref(self._ap),
                                                C.byref(h)), "uva_step_graph_create")
         self._h = h
 
