@@ -51,10 +51,14 @@ namespace {
 constexpr int kNB = 16;                  // block edge
 constexpr int kBE = kNB * kNB;           // elements of a block (one plane)
 constexpr int kMaxW = 15;                // blocks left of the diagonal: the groups of a CTA less one
-constexpr int kNT = 256;                 // threads: 16 groups of 16
+constexpr int kCT = 256;                 // compute threads: 16 groups of 16
+constexpr int kCW = kCT / 32;
+constexpr int kNT = kCT + 32;            // and one warp that feeds the solve's ring
 constexpr int kNW = kNT / 32;
+constexpr int kPitch = 20;               // pitch of a staged column: conflict-free m8n8k4 fragments
+constexpr int kSB = kNB * kPitch;        // doubles of a staged block (one plane)
 constexpr int kMaxBlk = kDirectMaxN / kNB;
-constexpr int kRing = 96 * 1024;         // bytes of staged factor blocks (2 CTAs per SM)
+constexpr int kRing = 94 * 1024;         // bytes of staged factor blocks (2 CTAs per SM)
 constexpr int kMaxStages = 8;
 constexpr int kLevelCap = 1024;          // vertices of one breadth-first level
 
@@ -148,9 +152,13 @@ __global__ void __launch_bounds__(kNT) k_band(uva_batch b) {
 // ------------------------------------------------------------------ small pieces
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
 
-__device__ __forceinline__ void mbar_init(unsigned bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kCT) : "memory"); }
 __device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -235,7 +243,7 @@ struct Isl {
     double2* rb;           // right-hand side / solution by band position
     double2 *y, *lu;       // A x of the last solution and of U, by solver row (ARAP)
     int stages;            // stages of the ring
-    unsigned step;         // solve steps so far (the ring's phase)
+    int q, ph;             // next stage and its phase (each thread its own: compute and feeding warps)
 };
 
 struct Shared {
@@ -243,10 +251,11 @@ struct Shared {
     int off[kMaxBlk + 1];                     // first block of each block row
     double red[2 * 4 * kNW];
     double dsm[2 * kNB * (kNB + 1)];          // S_KK (two planes, padded rows)
-    double dinv[2 * kBE];                     // D_K^-1 (swizzled)
+    double dinv[2 * kSB];                     // D_K^-1 (staged layout)
+    double2 prow[2][2][kNB], pcol[2][2][kNB]; // pivot rows and columns of the inversion
     double diag[kNB];                         // diagonal of A_KK
     double2 xk[2][kNB];                       // the block being substituted
-    unsigned long long bar[kMaxStages];
+    unsigned long long full[kMaxStages], empty[kMaxStages];
     int bad, rank, scan[kNW];
 };
 
@@ -283,7 +292,7 @@ __device__ __forceinline__ double2 apply(const uva_batch& b, const Isl& I, int i
 
 // ------------------------------------------------------------------ factor
 // acc (8 rows x 16 columns: two m8n8 tiles, CP: real then imaginary) +-=
-// A[8 mt ..][.] conj(B)^T for one block pair.
+// A[8 mt ..][.] conj(B)^T for one block pair, B in the staged layout.
 template <bool CP, bool SUB>
 __device__ __forceinline__ void block_mma(double (&acc)[CP ? 4 : 2][2], const double (&a)[4], const double (&ai)[CP ? 4 : 1],
                                           const double* B, int lane) {
@@ -295,11 +304,11 @@ __device__ __forceinline__ void block_mma(double (&acc)[CP ? 4 : 2][2], const do
         if constexpr (CP) aim = SUB ? -ai[ks] : ai[ks];
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
-            const int e = sw((lane >> 2) + 8 * nt, k);
+            const int e = k * kPitch + (lane >> 2) + 8 * nt;
             const double br = B[e];
             dmma(acc[nt], ar, br);
             if constexpr (CP) {
-                const double bi = B[kBE + e];
+                const double bi = B[kSB + e];
                 dmma(acc[nt], aim, bi);
                 dmma(acc[2 + nt], aim, br);
                 dmma(acc[2 + nt], -ar, bi);
@@ -368,66 +377,63 @@ __device__ void assemble(const uva_batch& b, const Isl& I, const Shared& S) {
     __syncthreads();
 }
 
-// D^-1 of the 16 x 16 (Hermitian) positive definite S_KK in S.dsm by one
-// warp: in-place Gauss-Jordan, two lanes per row with eight columns each.
-// Sets S.bad when a pivot is not above 1e-13 of A's diagonal.
+// D^-1 of the 16 x 16 (Hermitian) positive definite S_KK in S.dsm, one element
+// per thread: Gauss-Jordan with 2 x 2 pivots, whose rows and columns pass
+// through shared memory (one barrier per pivot pair). Into S.dinv and Dk. Sets
+// S.bad when a pivot is not above 1e-13 of A's diagonal.
 template <bool CP>
-__device__ __forceinline__ void invert_block(Shared& S, int lane) {
-    const int r = lane >> 1, h = lane & 1;
-    double w[8], wi[CP ? 8 : 1];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        w[j] = S.dsm[r * (kNB + 1) + 8 * h + j];
-        if constexpr (CP) wi[j] = S.dsm[kNB * (kNB + 1) + r * (kNB + 1) + 8 * h + j];
-    }
+__device__ __forceinline__ void invert_block(Shared& S, double* Dk) {
+    const int r = threadIdx.x >> 4, c = threadIdx.x & 15;
+    double2 w = make_double2(S.dsm[r * (kNB + 1) + c], CP ? S.dsm[kNB * (kNB + 1) + r * (kNB + 1) + c] : 0.0);
     bool bad = false;
+    auto mul = [](double2 x, double2 y) {
+        return CP ? make_double2(x.x * y.x - x.y * y.y, x.x * y.y + x.y * y.x) : make_double2(x.x * y.x, 0.0);
+    };
+    auto add = [](double2 x, double2 y) { return make_double2(x.x + y.x, CP ? x.y + y.y : 0.0); };
 #pragma unroll
-    for (int k = 0; k < kNB; ++k) {
-        const int kh = k >> 3, kj = k & 7;
-        const double piv = __shfl_sync(0xffffffffu, w[kj], 2 * k + kh);
-        bad |= !(piv > 1e-13 * S.diag[k]);
-        const double ip = 1.0 / piv;
-        const double f = __shfl_sync(0xffffffffu, w[kj], (lane & ~1) | kh);   // W[r][k]
-        double fi = 0.0;
-        if constexpr (CP) fi = __shfl_sync(0xffffffffu, wi[kj], (lane & ~1) | kh);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const bool isk = h == kh && j == kj;
-            double rk = __shfl_sync(0xffffffffu, w[j], 2 * k + h) * ip;
-            double rki = 0.0;
-            if constexpr (CP) rki = __shfl_sync(0xffffffffu, wi[j], 2 * k + h) * ip;
-            if (isk) { rk = ip; rki = 0.0; }
-            if (r == k) {
-                w[j] = rk;
-                if constexpr (CP) wi[j] = rki;
-            } else {
-                const double base = isk ? 0.0 : w[j];
-                if constexpr (CP) {
-                    const double bi = isk ? 0.0 : wi[j];
-                    w[j] = base - (f * rk - fi * rki);
-                    wi[j] = bi - (f * rki + fi * rk);
-                } else {
-                    w[j] = base - f * rk;
-                }
-            }
+    for (int k = 0; k < kNB; k += 2) {
+        double2(*row)[kNB] = S.prow[(k >> 1) & 1];
+        double2(*col)[kNB] = S.pcol[(k >> 1) & 1];
+        if ((r >> 1) == (k >> 1)) row[r & 1][c] = w;
+        if ((c >> 1) == (k >> 1)) col[c & 1][r] = w;
+        compute_sync();
+        const double a = row[0][k].x, d = row[1][k + 1].x;
+        const double2 b = row[0][k + 1];
+        const double det = a * d - (CP ? b.x * b.x + b.y * b.y : b.x * b.x);
+        bad |= !(a > 1e-13 * S.diag[k]) || !(det > 1e-13 * S.diag[k + 1] * a);
+        const double id = 1.0 / det;
+        const double2 p00 = make_double2(d * id, 0.0), p11 = make_double2(a * id, 0.0);
+        const double2 p01 = make_double2(-b.x * id, -b.y * id), p10 = make_double2(p01.x, -p01.y);
+        // the column's entry of the scaled pivot rows (its own columns: P^-1)
+        const bool pc = (c >> 1) == (k >> 1);
+        const double2 g0 = row[0][c], g1 = row[1][c];
+        double2 t0 = add(mul(p00, g0), mul(p01, g1)), t1 = add(mul(p10, g0), mul(p11, g1));
+        if (pc) { t0 = c & 1 ? p01 : p00; t1 = c & 1 ? p11 : p10; }
+        if ((r >> 1) == (k >> 1)) {
+            w = r & 1 ? t1 : t0;
+        } else {
+            const double2 u = add(mul(col[0][r], t0), mul(col[1][r], t1));
+            w = make_double2((pc ? 0.0 : w.x) - u.x, (pc ? 0.0 : w.y) - u.y);
         }
     }
-    if (bad && lane == 0) S.bad = 1;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int e = sw(r, 8 * h + j);
-        S.dinv[e] = w[j];
-        if constexpr (CP) S.dinv[kBE + e] = wi[j];
+    if (bad) S.bad = 1;
+    S.dinv[c * kPitch + r] = w.x;
+    Dk[sw(r, c)] = w.x;
+    if constexpr (CP) {
+        S.dinv[kSB + c * kPitch + r] = w.y;
+        Dk[kBE + sw(r, c)] = w.y;
     }
 }
 
-// Factor in place: on return block (K, K) holds D_K^-1 and (I, K) holds L_IK.
-// False when a pivot vanished.
+// Factor in place (the compute warps): on return block (K, K) holds D_K^-1 and
+// (I, K) holds L_IK; S.bad is set when a pivot vanished.
 template <Op OP>
-__device__ bool factor(const Isl& I, Shared& S, double* stage) {
+__device__ void factor(const Isl& I, Shared& S, double* stage) {
     constexpr bool CP = OP == OP_LSCM;
-    constexpr int BB = kBE * (CP ? 2 : 1);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int BB = kBE * (CP ? 2 : 1), SB = kSB * (CP ? 2 : 1);
+    constexpr int kAhead = 3;   // blocks of G whose loads are in flight together
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int sc = tid >> 4, sr = (tid & 15) ^ sc;   // the element at offset tid of a stored block
     for (int K = 0; K < I.nblk; ++K) {
         const int f = S.first[K], wl = K - f;
         // block rows below K that reach column K (first[] does not decrease)
@@ -435,15 +441,16 @@ __device__ bool factor(const Isl& I, Shared& S, double* stage) {
                                                               S.first[min(K + 1 + lane, kMaxBlk)] <= K));
         double* Lrow = I.L + static_cast<size_t>(S.off[K]) * BB;
         double* Dk = Lrow + static_cast<size_t>(wl) * BB;
-        {   // L_K. of the earlier columns into shared memory
-            const double2* src = reinterpret_cast<const double2*>(Lrow);
-            double2* dst = reinterpret_cast<double2*>(stage);
-            for (int k = threadIdx.x; k < wl * (BB / 2); k += kNT) dst[k] = src[k];
-            if (threadIdx.x < kNB) S.diag[threadIdx.x] = Dk[sw(threadIdx.x, threadIdx.x)];
+        // L_K. of the earlier columns into shared memory
+#pragma unroll 3
+        for (int k = 0; k < wl; ++k) {
+            stage[k * SB + sc * kPitch + sr] = Lrow[static_cast<size_t>(k) * BB + tid];
+            if constexpr (CP) stage[k * SB + kSB + sc * kPitch + sr] = Lrow[static_cast<size_t>(k) * BB + kBE + tid];
         }
-        __syncthreads();
+        if (tid < kNB) S.diag[tid] = Dk[sw(tid, tid)];
+        compute_sync();
         // S_IK for I = K .. K + cnt, half a block (8 rows) per task
-        for (int t = warp; t < 2 * (cnt + 1); t += kNW) {
+        for (int t = warp; t < 2 * (cnt + 1); t += kCW) {
             const int R = K + (t >> 1), mt = t & 1;
             double* blk = I.L + static_cast<size_t>(S.off[R] + K - S.first[R]) * BB;
             double acc[CP ? 4 : 2][2];
@@ -457,18 +464,14 @@ __device__ bool factor(const Isl& I, Shared& S, double* stage) {
                     if constexpr (CP) acc[2 + nt][u] = blk[kBE + e];
                 }
             const double* Gr = I.G + static_cast<size_t>((R & 15) * 16) * BB;
-            int M = S.first[R];
-            if (M < K) {
-                double a[4], ai[CP ? 4 : 1];
-                load_a<CP>(Gr + static_cast<size_t>(M & 15) * BB, mt, lane, a, ai);
-                for (; M < K; ++M) {
-                    double an[4], ani[CP ? 4 : 1];
-                    const int Mn = M + 1 < K ? M + 1 : M;   // next block's loads in flight
-                    load_a<CP>(Gr + static_cast<size_t>(Mn & 15) * BB, mt, lane, an, ani);
-                    block_mma<CP, true>(acc, a, ai, stage + (M - f) * BB, lane);
+            for (int M = S.first[R]; M < K; M += kAhead) {
+                double a[kAhead][4], ai[kAhead][CP ? 4 : 1];
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) { a[k] = an[k]; if constexpr (CP) ai[k] = ani[k]; }
-                }
+                for (int u = 0; u < kAhead; ++u)
+                    load_a<CP>(Gr + static_cast<size_t>(min(M + u, K - 1) & 15) * BB, mt, lane, a[u], ai[u]);
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u)
+                    if (M + u < K) block_mma<CP, true>(acc, a[u], ai[u], stage + (M + u - f) * SB, lane);
             }
             double* G = I.G + static_cast<size_t>((R & 15) * 16 + (K & 15)) * BB;
 #pragma unroll
@@ -485,12 +488,11 @@ __device__ bool factor(const Isl& I, Shared& S, double* stage) {
                     }
                 }
         }
-        __syncthreads();
-        if (warp == 0) invert_block<CP>(S, lane);
-        __syncthreads();
-        if (S.bad) return false;
-        for (int k = threadIdx.x; k < BB; k += kNT) Dk[k] = S.dinv[k];
-        for (int t = warp; t < 2 * cnt; t += kNW) {   // L_IK = S_IK D^-1
+        compute_sync();
+        invert_block<CP>(S, Dk);
+        compute_sync();
+        if (S.bad) return;
+        for (int t = warp; t < 2 * cnt; t += kCW) {   // L_IK = S_IK D^-1
             const int R = K + 1 + (t >> 1), mt = t & 1;
             double acc[CP ? 4 : 2][2] = {};
             double a[4], ai[CP ? 4 : 1];
@@ -507,18 +509,16 @@ __device__ bool factor(const Isl& I, Shared& S, double* stage) {
                     if constexpr (CP) blk[kBE + e] = acc[2 + nt][u];
                 }
         }
-        __syncthreads();
+        compute_sync();
     }
-    // the substitutions read the factor through the asynchronous proxy
-    asm volatile("fence.proxy.async;" ::: "memory");
-    __syncthreads();
-    return true;
 }
 
 // ------------------------------------------------------------------ solve
 // rb <- A^-1 rb. Group g = tid / 16 owns the block rows congruent to g: the
 // right-hand side of its current row stays in registers until the row is
-// final, then the group publishes it and takes the row 16 further on.
+// final, then the group publishes it and takes the row 16 further on. The
+// last warp feeds the ring: it copies a step's blocks once the compute warps
+// have released the stage.
 template <Op OP>
 __device__ void solve(Isl& I, Shared& S, double* stage) {
     constexpr bool CP = OP == OP_LSCM;
@@ -527,45 +527,53 @@ __device__ void solve(Isl& I, Shared& S, double* stage) {
     const int tid = threadIdx.x, lane = tid & 31, g = tid >> 4, r = tid & 15;
     const int nblk = I.nblk, NS = I.stages;
     const int stage_d = kRing / 8 / NS / 2 * 2;    // doubles per stage (16-byte multiple)
-    const unsigned bar0 = smem_addr(S.bar), st0 = smem_addr(stage);
-    const unsigned base = I.step;
-    auto fwd_issue = [&](int K) {   // warp 0: column K's blocks, one copy each
-        const unsigned q = (base + K) % NS, bar = bar0 + 8 * q, dst = st0 + q * stage_d * 8;
-        const int R = K + 1 + lane;
-        const bool on = lane < kMaxW && R < nblk && S.first[R] <= K;
-        const unsigned cnt = __popc(__ballot_sync(0xffffffffu, on));
-        if (lane == 0) mbar_expect(bar, cnt * kBytes);
-        __syncwarp();
-        if (on) bulk_copy(dst + lane * kBytes, I.L + static_cast<size_t>(S.off[R] + K - S.first[R]) * BB, kBytes, bar);
+    const unsigned full0 = smem_addr(S.full), empty0 = smem_addr(S.empty), st0 = smem_addr(stage);
+    int q = I.q, ph = I.ph;
+    auto next = [&]() {
+        if (++q == NS) { q = 0; ph ^= 1; }
     };
-    auto bwd_issue = [&](int K, int at) {   // row K's blocks are contiguous
-        const unsigned q = (base + at) % NS, bar = bar0 + 8 * q, dst = st0 + q * stage_d * 8;
-        const unsigned bytes = (K - S.first[K]) * kBytes;
-        if (lane == 0) {
-            mbar_expect(bar, bytes);
-            if (bytes) bulk_copy(dst, I.L + static_cast<size_t>(S.off[K]) * BB, bytes, bar);
+    if (tid >= kCT) {
+        for (int K = 0; K < nblk; ++K) {   // column K's blocks, one copy each
+            const int R = K + 1 + lane;
+            const bool on = lane < kMaxW && R < nblk && S.first[min(R, kMaxBlk)] <= K;
+            const unsigned cnt = __popc(__ballot_sync(0xffffffffu, on));
+            if (!mbar_wait(empty0 + 8 * q, ph ^ 1)) S.bad = 2;
+            if (lane == 0) mbar_expect(full0 + 8 * q, cnt * kBytes);
+            __syncwarp();
+            if (on)
+                bulk_copy(st0 + q * stage_d * 8 + lane * kBytes,
+                          I.L + static_cast<size_t>(S.off[R] + K - S.first[R]) * BB, kBytes, full0 + 8 * q);
+            next();
         }
-    };
-    // ---- forward: r_I -= L_IK r_K
-    if (tid < 32)
-        for (int K = 0; K < min(NS - 1, nblk); ++K) fwd_issue(K);
-    {
+        for (int K = nblk - 1; K >= 0; --K) {   // row K's blocks are contiguous
+            const unsigned bytes = (K - S.first[K]) * kBytes;
+            if (!mbar_wait(empty0 + 8 * q, ph ^ 1)) S.bad = 2;
+            if (lane == 0) {
+                mbar_expect(full0 + 8 * q, bytes);
+                if (bytes)
+                    bulk_copy(st0 + q * stage_d * 8, I.L + static_cast<size_t>(S.off[K]) * BB, bytes, full0 + 8 * q);
+            }
+            __syncwarp();
+            next();
+        }
+    } else {
+        // ---- forward: r_I -= L_IK r_K
         int R = g;
         double2 acc = R < nblk ? I.rb[R * kNB + r] : make_double2(0.0, 0.0);
         double2 nxt = R + 16 < nblk ? I.rb[(R + 16) * kNB + r] : make_double2(0.0, 0.0);
+        int fr = R < nblk ? S.first[R] : nblk;
         for (int K = 0; K < nblk; ++K) {
             if (R == K) {
                 S.xk[K & 1][r] = acc;
                 I.rb[K * kNB + r] = acc;
                 R += 16;
                 acc = nxt;
+                fr = R < nblk ? S.first[R] : nblk;
                 if (R + 16 < nblk) nxt = I.rb[(R + 16) * kNB + r];
             }
-            __syncthreads();   // r_K visible; the stage of step K - 1 is free
-            if (tid < 32 && K + NS - 1 < nblk) fwd_issue(K + NS - 1);
-            const unsigned at = base + K, q = at % NS;
-            if (!mbar_wait(bar0 + 8 * q, (at / NS) & 1)) S.bad = 2;
-            if (R < nblk && S.first[R] <= K) {
+            compute_sync();   // r_K visible
+            if (!mbar_wait(full0 + 8 * q, ph)) S.bad = 2;
+            if (fr <= K) {
                 const double* B = stage + q * stage_d + (R - K - 1) * BB;
                 const double2* x = S.xk[K & 1];
                 double ax = 0.0, ay = 0.0, bx = 0.0, by = 0.0;
@@ -584,54 +592,48 @@ __device__ void solve(Isl& I, Shared& S, double* stage) {
                 acc.x -= ax + bx;
                 acc.y -= ay + by;
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty0 + 8 * q);
+            next();
         }
-    }
-    __syncthreads();
-    // ---- z_K = D_K^-1 r_K, every block at once
-    for (int K0 = 0; K0 < nblk; K0 += kNT / 16) {   // the same trip count on both groups of a warp
-        const int K = min(K0 + g, nblk - 1);
-        const double* B = I.L + static_cast<size_t>(S.off[K + 1] - 1) * BB;
-        const double2 own = I.rb[K * kNB + r];
-        double zx = 0.0, zy = 0.0;
+        compute_sync();
+        // ---- z_K = D_K^-1 r_K, every block at once
+        for (int K0 = 0; K0 < nblk; K0 += kCT / 16) {   // the same trip count on both groups of a warp
+            const int K = min(K0 + g, nblk - 1);
+            const double* B = I.L + static_cast<size_t>(S.off[K + 1] - 1) * BB;
+            const double2 own = I.rb[K * kNB + r];
+            double zx = 0.0, zy = 0.0;
 #pragma unroll
-        for (int c = 0; c < kNB; ++c) {
-            const double l = B[sw(r, c)];
-            const double xx = __shfl_sync(0xffffffffu, own.x, c, 16), xy = __shfl_sync(0xffffffffu, own.y, c, 16);
-            zx += l * xx; zy += l * xy;
-            if constexpr (CP) {
-                const double m = B[kBE + sw(r, c)];
-                zx -= m * xy; zy += m * xx;
+            for (int c = 0; c < kNB; ++c) {
+                const double l = B[sw(r, c)];
+                const double xx = __shfl_sync(0xffffffffu, own.x, c, 16), xy = __shfl_sync(0xffffffffu, own.y, c, 16);
+                zx += l * xx; zy += l * xy;
+                if constexpr (CP) {
+                    const double m = B[kBE + sw(r, c)];
+                    zx -= m * xy; zy += m * xx;
+                }
             }
+            if (K0 + g < nblk) I.rb[K * kNB + r] = make_double2(zx, zy);
         }
-        if (K0 + g < nblk) I.rb[K * kNB + r] = make_double2(zx, zy);
-    }
-    __syncthreads();
-    // ---- backward: z_J -= L_KJ^H x_K
-    const unsigned half = nblk;   // steps of the ring used by the forward pass
-    if (tid < 32)
-        for (int t = 0; t < min(NS - 1, nblk); ++t) bwd_issue(nblk - 1 - t, half + t);
-    {
-        const int top = (nblk - 1 - g) & 15;          // the highest block row congruent to g
-        int J = nblk - 1 - top;
-        double2 acc = J >= 0 ? I.rb[J * kNB + r] : make_double2(0.0, 0.0);
-        double2 nxt = J - 16 >= 0 ? I.rb[(J - 16) * kNB + r] : make_double2(0.0, 0.0);
-        for (int t = 0; t < nblk; ++t) {
-            const int K = nblk - 1 - t;
+        compute_sync();
+        // ---- backward: z_J -= L_KJ^H x_K
+        int J = nblk - 1 - ((nblk - 1 - g) & 15);          // the highest block row congruent to g
+        acc = J >= 0 ? I.rb[J * kNB + r] : make_double2(0.0, 0.0);
+        nxt = J - 16 >= 0 ? I.rb[(J - 16) * kNB + r] : make_double2(0.0, 0.0);
+        for (int K = nblk - 1; K >= 0; --K) {
             if (J == K) {
-                S.xk[t & 1][r] = acc;
+                S.xk[K & 1][r] = acc;
                 I.rb[K * kNB + r] = acc;
                 J -= 16;
                 acc = nxt;
                 if (J - 16 >= 0) nxt = I.rb[(J - 16) * kNB + r];
             }
-            __syncthreads();
-            if (tid < 32 && t + NS - 1 < nblk) bwd_issue(nblk - 1 - (t + NS - 1), half + t + NS - 1);
-            const unsigned at = base + half + t, q = at % NS;
-            if (!mbar_wait(bar0 + 8 * q, (at / NS) & 1)) S.bad = 2;
             const int f = S.first[K];
+            compute_sync();
+            if (!mbar_wait(full0 + 8 * q, ph)) S.bad = 2;
             if (J >= f) {   // J < K
                 const double* B = stage + q * stage_d + (J - f) * BB;
-                const double2* x = S.xk[t & 1];
+                const double2* x = S.xk[K & 1];
                 double ax = 0.0, ay = 0.0, bx = 0.0, by = 0.0;
 #pragma unroll
                 for (int c = 0; c < kNB; c += 2) {
@@ -648,9 +650,13 @@ __device__ void solve(Isl& I, Shared& S, double* stage) {
                 acc.x -= ax + bx;
                 acc.y -= ay + by;
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty0 + 8 * q);
+            next();
         }
     }
-    I.step = base + 2 * nblk;
+    I.q = q;
+    I.ph = ph;
     __syncthreads();
 }
 
@@ -886,7 +892,7 @@ __global__ void __launch_bounds__(kNT, 2) k_direct(uva_batch b, uva_solve_params
             I.lu = I.y + npad;
             const int w = max(info[2], 1);
             I.stages = max(1, min(kMaxStages, kRing / (w * BB * 8)));
-            I.step = 0;
+            I.q = I.ph = 0;
             // skyline and block offsets
             constexpr int kPer = (kMaxBlk + kNT - 1) / kNT;
             int sum = 0, fs[kPer];
@@ -904,7 +910,10 @@ __global__ void __launch_bounds__(kNT, 2) k_direct(uva_batch b, uva_solve_params
             }
             if ((tid & 31) == 31) S.scan[tid >> 5] = inc;
             if (tid == 0) S.bad = 0;
-            if (tid < I.stages) mbar_init(smem_addr(S.bar + tid));
+            if (tid < I.stages) {
+                mbar_init(smem_addr(S.full + tid), 1);
+                mbar_init(smem_addr(S.empty + tid), kCW);
+            }
             __syncthreads();
             int at = inc - sum;
             for (int k = 0; k < (tid >> 5); ++k) at += S.scan[k];
@@ -927,14 +936,21 @@ __global__ void __launch_bounds__(kNT, 2) k_direct(uva_batch b, uva_solve_params
                 done = true;
             } else {
                 assemble<OP>(b, I, S);
-                if (factor<OP>(I, S, stage)) {
+                if (tid < kCT) factor<OP>(I, S, stage);
+                // the substitutions read the factor through the asynchronous proxy
+                asm volatile("fence.proxy.async;" ::: "memory");
+                __syncthreads();
+                if (S.bad == 0) {
                     if (CP) done = solve_lscm(b, prm, I, S, rd, stage);
                     else done = solve_arap(b, prm, I, S, rd, stage);
                     if (S.bad) done = false;
                 }
             }
             __syncthreads();
-            if (tid < I.stages) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(S.bar + tid)) : "memory");
+            if (tid < I.stages) {
+                asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(S.full + tid)) : "memory");
+                asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(S.empty + tid)) : "memory");
+            }
         }
         if (tid == 0) {
             info[3] = done ? 1 : 0;
@@ -943,7 +959,7 @@ __global__ void __launch_bounds__(kNT, 2) k_direct(uva_batch b, uva_solve_params
                 st.t_begin = t0;
                 st.t_end = global_ns();
                 st.sm = static_cast<int32_t>(sm_id());
-                st.team = kNT;
+                st.team = kCT;
             } else {
                 atomicAdd(b.work + kWorkLeft, 1);
             }
