@@ -3,12 +3,14 @@
 //
 //  * k_tri_jacobians: closed-form 2x2 singular values of the 3D->UV Jacobian
 //    (metrics.py:115-145), signed UV area, 3D area, angle error (:213-223).
-//  * reductions: FP64 sums (warp-reduced, then atomics) of the report terms.
-//  * weighted quantiles (metrics.py:107-112, param.py:543-546): a segmented
-//    weighted radix select over the FP64 bit patterns, 8 bits per pass,
-//    returning the smallest value whose cumulative weight reaches q * total
-//    (numpy: argsort, cumsum, searchsorted). One segment for the whole mesh,
-//    or one per island for batched chart quality.
+//  * reductions: FP64 sums of the report terms, per thread over many triangles,
+//    then per block, then one atomic per block and term.
+//  * weighted quantiles (metrics.py:107-112, param.py:543-546): a weighted
+//    radix select over the FP64 bit patterns, 8 bits per pass, returning the
+//    smallest value whose cumulative weight reaches q * total (numpy: argsort,
+//    cumsum, searchsorted). The report's quantiles share eight launches
+//    (k_qsel), an island's takes one CTA (k_q_island), and arbitrary segments
+//    keep global histograms (k_q_hist).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -79,43 +81,81 @@ __device__ __forceinline__ void load_corners(const double* V, const double* UV, 
     }
 }
 
-template <int K>
-__device__ __forceinline__ void warp_atomic_sums(double* dst, double (&v)[K]) {
+// Block sums of K values per thread, then one atomic per block and value (one
+// per warp contended: 14 addresses took 55,000 atomics each on 1.8M triangles).
+template <int NT, int K>
+__device__ __forceinline__ void block_atomic_sums(double* dst, double (&v)[K]) {
+    __shared__ double part[NT / 32][K];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+        if (lane == 0) part[warp][k] = v[k];
     }
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int k = 0; k < K; ++k)
-            if (v[k] != 0.0) atomicAdd(dst + k, v[k]);
+    __syncthreads();
+    if (threadIdx.x < K) {
+        double t = 0.0;
+        for (int w = 0; w < NT / 32; ++w) t += part[w][threadIdx.x];
+        if (t != 0.0) atomicAdd(dst + threadIdx.x, t);
     }
 }
 
-// Pass A: per-triangle values; global sums of a3 and |sa|; per-island a3,
-// |sa|, positive / negative 3D area (metrics.py:160-200).
-__global__ void k_met_a(int m, const double* V, const double* UV, const int32_t* F, const int32_t* isl, double* tri,
-                        double* sums, double* isum) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    double v[2] = {0.0, 0.0};
-    if (t < m) {
-        double P[9], U[6];
-        load_corners(V, UV, F, t, P, U);
-        const TriJ r = tri_jacobian(P, U);
-        double* o = tri + 6 * static_cast<size_t>(t);
-        o[0] = r.s1; o[1] = r.s2; o[2] = r.sa; o[3] = r.a3; o[4] = r.good ? 1.0 : 0.0; o[5] = r.ang;
-        v[0] = r.a3;
-        v[1] = fabs(r.sa);
-        if (isl) {
-            double* s = isum + 4 * static_cast<size_t>(isl[t]);
-            atomicAdd(s, r.a3);
-            atomicAdd(s + 1, fabs(r.sa));
-            if (r.sa > 0.0) atomicAdd(s + 2, r.a3);
-            if (r.sa < 0.0) atomicAdd(s + 3, r.a3);
+// Sums of K values over the runs of equal keys along a warp (key -1: none),
+// then one atomic per run and value at dst + stride * key. Keys may come in
+// any order: a run is what is contiguous. Every lane calls.
+template <int K>
+__device__ __forceinline__ void warp_run_sums(double* dst, int stride, int key, double (&v)[K]) {
+    const int lane = threadIdx.x & 31;
+    const int prev = __shfl_up_sync(0xffffffffu, key, 1);
+    const bool head = lane == 0 || prev != key;
+    const unsigned heads = __ballot_sync(0xffffffffu, head);
+    const unsigned above = lane == 31 ? 0u : heads & (0xfffffffeu << lane);
+    const int end = above ? __ffs(above) - 1 : 32;    // one past the run's last lane
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const double y = __shfl_down_sync(0xffffffffu, v[k], o);
+            if (lane + o < end) v[k] += y;
         }
     }
-    warp_atomic_sums<2>(sums, v);
+    if (key >= 0 && head) {
+        double* d = dst + static_cast<size_t>(stride) * key;
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (v[k] != 0.0) atomicAdd(d + k, v[k]);
+    }
+}
+
+constexpr int kMetNT = 256;   // threads of the report passes, a few blocks per SM
+
+// Pass A: per-triangle values; global sums of a3 and |sa|; per-island a3,
+// |sa|, positive / negative 3D area (metrics.py:160-200).
+__global__ void __launch_bounds__(kMetNT) k_met_a(int m, const double* V, const double* UV, const int32_t* F,
+                                                  const int32_t* isl, double* tri, double* sums, double* isum) {
+    double v[2] = {0.0, 0.0};
+    for (int t0 = blockIdx.x * kMetNT; t0 < m; t0 += gridDim.x * kMetNT) {   // uniform over the block
+        const int t = t0 + threadIdx.x;
+        int key = -1;
+        double s4[4] = {0.0, 0.0, 0.0, 0.0};
+        if (t < m) {
+            double P[9], U[6];
+            load_corners(V, UV, F, t, P, U);
+            const TriJ r = tri_jacobian(P, U);
+            double* o = tri + 6 * static_cast<size_t>(t);
+            o[0] = r.s1; o[1] = r.s2; o[2] = r.sa; o[3] = r.a3; o[4] = r.good ? 1.0 : 0.0; o[5] = r.ang;
+            v[0] += r.a3;
+            v[1] += fabs(r.sa);
+            if (isl) key = isl[t];
+            s4[0] = r.a3;
+            s4[1] = fabs(r.sa);
+            s4[2] = r.sa > 0.0 ? r.a3 : 0.0;
+            s4[3] = r.sa < 0.0 ? r.a3 : 0.0;
+        }
+        if (isl) warp_run_sums<4>(isum, 4, key, s4);
+    }
+    block_atomic_sums<kMetNT, 2>(sums, v);
 }
 
 // Quantile inputs: value (excluded: +inf) and weight (excluded: 0).
@@ -126,11 +166,10 @@ struct QIn {
 
 // Pass B (metrics.py:160-205): report sums and the quantile inputs.
 // sums layout: 0 sum a3, 1 sum |sa|, 2.. see UVA_MET_* in the host code.
-__global__ void k_met_b(int m, const double* tri, const int32_t* isl, const double* isum, double* sums, QIn qa, QIn qg,
-                        QIn qc) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kMetNT) k_met_b(int m, const double* tri, const int32_t* isl, const double* isum,
+                                                  double* sums, QIn qa, QIn qg, QIn qc) {
     double v[14] = {0};
-    if (t < m) {
+    for (int t = blockIdx.x * kMetNT + threadIdx.x; t < m; t += gridDim.x * kMetNT) {
         const double* o = tri + 6 * static_cast<size_t>(t);
         const double s1 = o[0], s2 = o[1], sa = o[2], a3 = o[3], ang = o[5];
         const bool good = o[4] != 0.0;
@@ -146,15 +185,15 @@ __global__ void k_met_b(int m, const double* tri, const int32_t* isl, const doub
         const double lg = fabs(log2(fmax(ar_g, 1e-30)));
         const bool ok = valid && !collapsed;
         const double st = sqrt((s1 * s1 + s2 * s2) / 2.0) / sqrt(fmax(scale2, 1e-300));
-        v[0] = collapsed ? 1.0 : 0.0;
-        v[1] = collapsed ? w : 0.0;
-        v[2] = an_ok ? aniso * w : 0.0;
-        v[3] = an_ok ? w : 0.0;
-        v[4] = valid ? ang * w : 0.0;
-        v[5] = valid ? w : 0.0;
-        v[6] = ok ? lg * w : 0.0;
-        v[7] = ok ? w : 0.0;
-        v[8] = ok ? st * st * w : 0.0;
+        v[0] += collapsed ? 1.0 : 0.0;
+        v[1] += collapsed ? w : 0.0;
+        v[2] += an_ok ? aniso * w : 0.0;
+        v[3] += an_ok ? w : 0.0;
+        v[4] += valid ? ang * w : 0.0;
+        v[5] += valid ? w : 0.0;
+        v[6] += ok ? lg * w : 0.0;
+        v[7] += ok ? w : 0.0;
+        v[8] += ok ? st * st * w : 0.0;
         qa.x[t] = an_ok ? aniso : INFINITY; qa.w[t] = an_ok ? w : 0.0;
         qg.x[t] = ok ? lg : INFINITY; qg.w[t] = ok ? w : 0.0;
         if (isl) {
@@ -165,13 +204,13 @@ __global__ void k_met_b(int m, const double* tri, const int32_t* isl, const doub
             const double dom = s[2] >= s[3] ? 1.0 : -1.0;
             const double sg = sa > 0.0 ? 1.0 : (sa < 0.0 ? -1.0 : (sa == 0.0 ? 0.0 : NAN));
             const bool flipped = valid && !collapsed && !(sg == dom);
-            v[9] = ok ? lc * w : 0.0;
-            v[10] = flipped ? 1.0 : 0.0;
-            v[11] = flipped ? w : 0.0;
+            v[9] += ok ? lc * w : 0.0;
+            v[10] += flipped ? 1.0 : 0.0;
+            v[11] += flipped ? w : 0.0;
             qc.x[t] = ok ? lc : INFINITY; qc.w[t] = ok ? w : 0.0;
         }
     }
-    warp_atomic_sums<14>(sums + 2, v);
+    block_atomic_sums<kMetNT, 14>(sums + 2, v);
 }
 
 // Per-island inputs of island_density_ratio_p95 and the mirrored count.
@@ -188,35 +227,10 @@ __global__ void k_met_islands(int ni, const double* isum, double* sums, QIn qd) 
         v[0] = s[2] >= s[3] ? 0.0 : 1.0;
         v[1] = s[0];
     }
-    warp_atomic_sums<2>(sums + 16, v);
+    block_atomic_sums<kMetNT, 2>(sums + 16, v);
 }
 
 // ------------------------------------------------------------------ chart quality
-// Per-key sums of K values over a warp whose lanes hold their keys in
-// contiguous runs (key -1: none): a segmented reduction, then the first lane
-// of each run adds the run's sums at dst + stride * key. Batch triangles are
-// grouped by island, so an island takes one atomic per value and warp.
-template <int K>
-__device__ __forceinline__ void warp_run_sums(double* dst, int stride, int key, double (&v)[K]) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int yk = __shfl_down_sync(0xffffffffu, key, o);
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const double y = __shfl_down_sync(0xffffffffu, v[k], o);
-            if (lane + o < 32 && yk == key) v[k] += y;
-        }
-    }
-    const int prev = __shfl_up_sync(0xffffffffu, key, 1);
-    if (key >= 0 && (lane == 0 || prev != key)) {
-        double* d = dst + static_cast<size_t>(stride) * key;
-#pragma unroll
-        for (int k = 0; k < K; ++k)
-            if (v[k] != 0.0) atomicAdd(d + k, v[k]);
-    }
-}
-
 // engine/param.py:520-551 for every island of a batch (frames from the setup).
 __global__ void k_quality_a(const uva_batch b, double* tri, double* isum) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -252,25 +266,30 @@ __global__ void k_quality_a(const uva_batch b, double* tri, double* isum) {
 __global__ void k_quality_b(const uva_batch b, const double* tri, double* isum, QIn qa, QIn qr, double* per_aniso,
                             double* per_area, double* stretch) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= b.t) return;
-    const int isl = reinterpret_cast<const int4*>(b.tri4)[f].w;
-    const double* o = tri + 6 * static_cast<size_t>(f);
-    double* s = isum + 8 * static_cast<size_t>(isl);
-    const double A = s[0];
-    const double sc = s[1] / fmax(A, 1e-300);
-    const double w = o[3] / fmax(A, 1e-300);
-    const double s1 = o[0], s2 = o[1];
-    const double an = s1 / fmax(s2, 1e-12);
-    const double ar = (s1 * s2) / fmax(sc, 1e-300);
-    const double lar = fabs(log2(fmax(ar, 1e-12)));
-    const double st2 = (s1 * s1 + s2 * s2) / 2.0 / fmax(sc, 1e-300);
-    per_aniso[f] = an;
-    per_area[f] = ar;
-    qa.x[f] = an; qa.w[f] = w;
-    qr.x[f] = lar; qr.w[f] = w;
-    atomicAdd(s + 6, an * w);
-    atomicAdd(s + 7, lar * w);
-    atomicAdd(stretch + isl, st2 * w);
+    int isl = -1;
+    double v[2] = {0.0, 0.0}, st[1] = {0.0};
+    if (f < b.t) {
+        isl = reinterpret_cast<const int4*>(b.tri4)[f].w;
+        const double* o = tri + 6 * static_cast<size_t>(f);
+        const double* s = isum + 8 * static_cast<size_t>(isl);
+        const double A = s[0];
+        const double sc = s[1] / fmax(A, 1e-300);
+        const double w = o[3] / fmax(A, 1e-300);
+        const double s1 = o[0], s2 = o[1];
+        const double an = s1 / fmax(s2, 1e-12);
+        const double ar = (s1 * s2) / fmax(sc, 1e-300);
+        const double lar = fabs(log2(fmax(ar, 1e-12)));
+        const double st2 = (s1 * s1 + s2 * s2) / 2.0 / fmax(sc, 1e-300);
+        per_aniso[f] = an;
+        per_area[f] = ar;
+        qa.x[f] = an; qa.w[f] = w;
+        qr.x[f] = lar; qr.w[f] = w;
+        v[0] = an * w;
+        v[1] = lar * w;
+        st[0] = st2 * w;
+    }
+    warp_run_sums<2>(isum + 6, 8, isl, v);
+    warp_run_sums<1>(stretch, 1, isl, st);
 }
 
 // Per island: flips, aniso_p95, aniso_mean, area_p95, area_logdev, stretch, scale, A.
@@ -297,6 +316,165 @@ __device__ __forceinline__ unsigned long long okey(double x) {
     return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
 }
 
+// ---- one or several whole arrays at once (the report)
+// One launch per 8-bit digit, every array at blockIdx.y. A thread sums a run of
+// equal digits before it touches the block's shared histogram (the leading
+// digits are all alike), blocks store their histograms, and the last block of
+// an array adds them in order and picks the digit: the same bits on every run.
+// 1.8M values, three arrays: 0.2 ms; one global FP64 atomic per value on 256
+// addresses took 15.9 ms.
+constexpr int kSelNT = 512, kSelBlocks = 148, kSelMax = 4;
+
+struct QSel {
+    const double *x[kSelMax], *w[kSelMax];
+    double* out[kSelMax];
+    int n[kSelMax];
+};
+struct QOne {
+    unsigned long long prefix;
+    double below, target, total;
+    unsigned ticket, done;
+};
+
+// The first digit whose cumulative weight reaches the target; if rounding
+// leaves the target above the total, the last non-empty one (numpy clamps to
+// the last element). -1: empty. c: the weight below the digit.
+__device__ __forceinline__ int pick_digit(const double* h, double target, double& c) {
+    int last = -1;
+    double clast = c;
+    for (int k = 0; k < 256; ++k) {
+        if (h[k] == 0.0) continue;
+        if (c + h[k] >= target) return k;
+        clast = c;
+        c += h[k];
+        last = k;
+    }
+    c = clast;
+    return last;
+}
+
+// Histogram of the digit below bit `hi` over elements i0, i0 + step, ... < n
+// whose bits from `hi` up equal the prefix's, added to the shared h.
+__device__ __forceinline__ void add_digits(const double* x, const double* w, int i0, int n, int step, int hi,
+                                           unsigned long long prefix, double* h) {
+    int cur = -1;
+    double acc = 0.0;
+    for (int i = i0; i < n; i += step) {
+        const double wi = w[i];
+        if (wi == 0.0) continue;
+        const unsigned long long k = okey(x[i]);
+        if (hi < 64 && (k >> hi) != (prefix >> hi)) continue;
+        const int d = static_cast<int>((k >> (hi - 8)) & 0xff);
+        if (d != cur) {
+            if (cur >= 0) atomicAdd(h + cur, acc);
+            cur = d;
+            acc = 0.0;
+        }
+        acc += wi;
+    }
+    // the last runs: one addition per warp where its lanes agree
+    const int d0 = __shfl_sync(0xffffffffu, cur, 0);
+    if (__all_sync(0xffffffffu, cur == d0)) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if ((threadIdx.x & 31) == 0 && d0 >= 0) atomicAdd(h + d0, acc);
+    } else if (cur >= 0) {
+        atomicAdd(h + cur, acc);
+    }
+}
+
+__device__ __forceinline__ double okey_value(unsigned long long k) {
+    return __longlong_as_double(static_cast<long long>((k >> 63) ? (k & 0x7fffffffffffffffull) : ~k));
+}
+
+__global__ void __launch_bounds__(kSelNT) k_qsel(QSel p, QOne* st, double* part, double q, int pass) {
+    __shared__ double h[256];
+    __shared__ unsigned turn;
+    const int a = blockIdx.y;
+    QOne* s = st + a;
+    const int hi = 64 - 8 * pass;
+    if (threadIdx.x < 256) h[threadIdx.x] = 0.0;
+    __syncthreads();
+    if (pass == 0 || !s->done)
+        add_digits(p.x[a], p.w[a], blockIdx.x * kSelNT + threadIdx.x, p.n[a], kSelBlocks * kSelNT, hi,
+                   pass ? s->prefix : 0, h);
+    __syncthreads();
+    double* mine = part + (static_cast<size_t>(a) * kSelBlocks + blockIdx.x) * 256;
+    if (threadIdx.x < 256) mine[threadIdx.x] = h[threadIdx.x];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) turn = atomicAdd(&s->ticket, 1u);
+    __syncthreads();
+    if (turn != kSelBlocks - 1) return;
+    __threadfence();
+    if (threadIdx.x < 256) {
+        const double* all = part + static_cast<size_t>(a) * kSelBlocks * 256 + threadIdx.x;
+        double t = 0.0;
+#pragma unroll 4
+        for (int b = 0; b < kSelBlocks; ++b) t += __ldcg(all + 256 * b);
+        h[threadIdx.x] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    s->ticket = 0;
+    if (pass == 0) {
+        double t = 0.0;
+        for (int k = 0; k < 256; ++k) t += h[k];
+        s->total = t;
+        s->target = q * t;
+        s->below = 0.0;
+        s->prefix = 0;
+        s->done = 0;
+    }
+    if (s->done) return;
+    double c = s->below;
+    const int d = pick_digit(h, s->target, c);
+    if (d < 0) {
+        s->done = 1;
+        *p.out[a] = NAN;
+        return;
+    }
+    s->below = c;
+    s->prefix |= static_cast<unsigned long long>(d) << (hi - 8);
+    if (hi == 8) *p.out[a] = s->total > 0.0 ? okey_value(s->prefix) : NAN;
+}
+
+// ---- one quantile per island of a batch (triangles [tofs[i], tofs[i + 1])),
+// a CTA per island and array: every digit in one launch.
+__global__ void __launch_bounds__(256) k_q_island(const int32_t* tofs, const double* x0, const double* w0, double* out0,
+                                                  const double* x1, const double* w1, double* out1, double q) {
+    __shared__ double h[256];
+    __shared__ unsigned long long prefix;
+    __shared__ int empty;
+    const int isl = blockIdx.x;
+    const double* x = blockIdx.y ? x1 : x0;
+    const double* w = blockIdx.y ? w1 : w0;
+    const int lo = tofs[isl], hi_t = tofs[isl + 1];
+    double below = 0.0, target = 0.0, total = 0.0;   // thread 0
+    if (threadIdx.x == 0) { prefix = 0; empty = 0; }
+    for (int hi = 64; hi > 0; hi -= 8) {
+        h[threadIdx.x] = 0.0;
+        __syncthreads();
+        // every warp makes the same number of trips as its lanes vote at the end
+        add_digits(x, w, lo + threadIdx.x, hi_t, 256, hi, prefix, h);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (hi == 64) {
+                for (int k = 0; k < 256; ++k) total += h[k];
+                target = q * total;
+            }
+            double c = below;
+            const int d = pick_digit(h, target, c);
+            if (d < 0) empty = 1;
+            else { below = c; prefix |= static_cast<unsigned long long>(d) << (hi - 8); }
+        }
+        __syncthreads();
+        if (empty) break;
+    }
+    if (threadIdx.x == 0) (blockIdx.y ? out1 : out0)[isl] = !empty && total > 0.0 ? okey_value(prefix) : NAN;
+}
+
+// ---- arbitrary segments (uva_wquantile with a segment array)
 struct QState {
     unsigned long long prefix;   // fixed high bits so far
     double below;                // weight of elements with key < prefix range
@@ -339,9 +517,6 @@ __global__ void k_q_hist(int n, const double* x, const double* w, const int32_t*
     atomicAdd(hist + 256 * static_cast<size_t>(s) + digit, wi);
 }
 
-// Pick the digit whose cumulative weight reaches the target: the first
-// bucket with below + cumsum >= target; if rounding leaves the target above
-// the total, the last non-empty bucket (numpy clamps to the last element).
 __global__ void k_q_pick(int ns, QState* st, double* hist) {
     const int s = blockIdx.x;
     if (s >= ns) return;
@@ -353,20 +528,9 @@ __global__ void k_q_pick(int ns, QState* st, double* hist) {
     if (threadIdx.x != 0) return;
     QState q = st[s];
     if (q.done || q.shift <= 0) return;
-    double c = q.below, clast = q.below;
-    int d = -1, last = -1;
-    for (int k = 0; k < 256; ++k) {
-        if (h[k] == 0.0) continue;
-        if (c + h[k] >= q.target) { d = k; break; }
-        clast = c;
-        c += h[k];
-        last = k;
-    }
-    if (d < 0) {
-        if (last < 0) { q.done = 1; st[s] = q; return; }
-        d = last;
-        c = clast;
-    }
+    double c = q.below;
+    const int d = pick_digit(h, q.target, c);
+    if (d < 0) { q.done = 1; st[s] = q; return; }
     q.below = c;
     q.prefix |= static_cast<unsigned long long>(d) << (q.shift - 8);
     q.shift -= 8;
@@ -378,10 +542,7 @@ __global__ void k_q_value(int ns, const QState* st, double* out) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= ns) return;
     const QState q = st[s];
-    unsigned long long k = q.prefix;
-    // invert okey
-    const unsigned long long u = (k >> 63) ? (k & 0x7fffffffffffffffull) : ~k;
-    out[s] = q.total > 0.0 ? __longlong_as_double(static_cast<long long>(u)) : NAN;
+    out[s] = q.total > 0.0 ? okey_value(q.prefix) : NAN;
 }
 
 size_t al(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
@@ -410,11 +571,23 @@ int wquantile(int n, const double* x, const double* w, const int32_t* seg, int s
 
 size_t wq_bytes(int ns) { return al(sizeof(double) * 256 * ns) + al(sizeof(QState) * ns) + al(sizeof(double) * ns); }
 
+// Quantiles of `count` whole arrays; scratch: qsel_bytes(count).
+size_t qsel_bytes(int count) { return al(sizeof(QOne) * kSelMax) + sizeof(double) * 256 * kSelBlocks * count; }
+
+int qselect(const QSel& p, int count, double q, unsigned char* scratch, cudaStream_t s) {
+    QOne* st = reinterpret_cast<QOne*>(scratch);
+    double* part = reinterpret_cast<double*>(scratch + al(sizeof(QOne) * kSelMax));
+    cudaMemsetAsync(st, 0, sizeof(QOne) * kSelMax, s);
+    for (int pass = 0; pass < 8; ++pass) k_qsel<<<dim3(kSelBlocks, count), kSelNT, 0, s>>>(p, st, part, q, pass);
+    UVA_CHECK_LAUNCH("uva_wquantile");
+    return UVA_OK;
+}
+
 }  // namespace
 
 extern "C" int uva_wquantile_scratch_bytes(int32_t nseg, int64_t* bytes) {
     if (nseg < 1 || !bytes) { uva_set_error("uva_wquantile_scratch_bytes: bad arguments"); return UVA_E_ARG; }
-    *bytes = static_cast<int64_t>(wq_bytes(nseg));
+    *bytes = static_cast<int64_t>(nseg == 1 ? std::max(wq_bytes(1), qsel_bytes(1)) : wq_bytes(nseg));
     return UVA_OK;
 }
 
@@ -422,6 +595,10 @@ extern "C" int uva_wquantile(const double* x, const double* w, const int32_t* se
                              double* out, void* scratch, int64_t scratch_bytes, void* stream) {
     if (n < 0 || nseg < 1 || !out || !scratch || (n > 0 && (!x || !w))) { uva_set_error("uva_wquantile: bad arguments"); return UVA_E_ARG; }
     if (scratch_bytes < static_cast<int64_t>(wq_bytes(nseg))) { uva_set_error("uva_wquantile: scratch too small"); return UVA_E_ARG; }
+    if (!seg && nseg == 1 && scratch_bytes >= static_cast<int64_t>(qsel_bytes(1))) {
+        const QSel p{{x}, {w}, {out}, {n}};
+        return qselect(p, 1, q, static_cast<unsigned char*>(scratch), static_cast<cudaStream_t>(stream));
+    }
     return wquantile(n, x, w, seg, 1, nseg, q, out, static_cast<unsigned char*>(scratch), static_cast<cudaStream_t>(stream));
 }
 
@@ -429,7 +606,7 @@ extern "C" int uva_metrics_scratch_bytes(int64_t m, int64_t n_islands, int64_t* 
     if (m < 0 || n_islands < 0 || !bytes) { uva_set_error("uva_metrics_scratch_bytes: bad arguments"); return UVA_E_ARG; }
     const int64_t ni = std::max<int64_t>(n_islands, 1);
     *bytes = static_cast<int64_t>(al(48 * std::max<int64_t>(m, 1)) + al(32 * ni) + 6 * al(8 * std::max<int64_t>(m, 1)) +
-                                  2 * al(8 * ni) + wq_bytes(std::max<int64_t>(ni, 1)) + al(8 * 64));
+                                  2 * al(8 * ni) + al(qsel_bytes(kSelMax)) + al(8 * 64));
     return UVA_OK;
 }
 
@@ -456,28 +633,25 @@ extern "C" int uva_distortion_report(const double* V, const double* UV, const in
     QIn qc{reinterpret_cast<double*>(base), reinterpret_cast<double*>(base + al(8 * M))}; base += 2 * al(8 * M);
     QIn qd{reinterpret_cast<double*>(base), reinterpret_cast<double*>(base + al(8 * static_cast<size_t>(ni)))};
     base += 2 * al(8 * static_cast<size_t>(ni));
-    unsigned char* wqs = base; base += wq_bytes(ni);
+    unsigned char* wqs = base; base += al(qsel_bytes(kSelMax));
     double* sums = reinterpret_cast<double*>(base);   // 64 doubles
     cudaMemsetAsync(sums, 0, 8 * 64, s);
     cudaMemsetAsync(isum, 0, 32 * static_cast<size_t>(ni), s);
-    const int tb = 256, gb = std::max(1, (m + tb - 1) / tb);
+    const int tb = kMetNT, gb = std::max(1, std::min((m + tb - 1) / tb, 148 * 6));
     k_met_a<<<gb, tb, 0, s>>>(m, V, UV, F, islands, tri, sums, isum);
     k_met_b<<<gb, tb, 0, s>>>(m, tri, islands, isum, sums, qa, qg, qc);
     if (islands) k_met_islands<<<(ni + tb - 1) / tb, tb, 0, s>>>(ni, isum, sums, qd);
     UVA_CHECK_LAUNCH("uva_distortion_report");
     // sums: [0] a3, [1] |sa|, [2..15] k_met_b terms, [16] mirrored, [17] ia3 total
     cudaMemcpyAsync(out, sums, sizeof(double) * 24, cudaMemcpyDeviceToDevice, s);
-    int rc = wquantile(m, qa.x, qa.w, nullptr, 1, 1, 0.95, out + 24, wqs, s);
-    if (rc == UVA_OK) rc = wquantile(m, qg.x, qg.w, nullptr, 1, 1, 0.95, out + 25, wqs, s);
-    if (rc == UVA_OK && islands) rc = wquantile(m, qc.x, qc.w, nullptr, 1, 1, 0.95, out + 26, wqs, s);
-    if (rc == UVA_OK && islands) rc = wquantile(ni, qd.x, qd.w, nullptr, 1, 1, 0.95, out + 27, wqs, s);
-    return rc;
+    const QSel p{{qa.x, qg.x, qc.x, qd.x}, {qa.w, qg.w, qc.w, qd.w}, {out + 24, out + 25, out + 26, out + 27}, {m, m, m, ni}};
+    return qselect(p, islands ? 4 : 2, 0.95, wqs, s);
 }
 
 extern "C" int uva_quality_scratch_bytes(int64_t t, int64_t nc, int64_t* bytes) {
     if (t < 0 || nc < 0 || !bytes) { uva_set_error("uva_quality_scratch_bytes: bad arguments"); return UVA_E_ARG; }
     const size_t T = std::max<int64_t>(t, 1), C = std::max<int64_t>(nc, 1);
-    *bytes = static_cast<int64_t>(al(48 * T) + al(64 * C) + 4 * al(8 * T) + 3 * al(8 * C) + wq_bytes(static_cast<int>(C)));
+    *bytes = static_cast<int64_t>(al(48 * T) + al(64 * C) + 4 * al(8 * T) + 3 * al(8 * C));
     return UVA_OK;
 }
 
@@ -503,18 +677,14 @@ extern "C" int uva_chart_quality(const uva_batch* b, double* out, double* per_an
     QIn qr{reinterpret_cast<double*>(base), reinterpret_cast<double*>(base + al(8 * T))}; base += 2 * al(8 * T);
     double* stretch = reinterpret_cast<double*>(base); base += al(8 * C);
     double* q95a = reinterpret_cast<double*>(base); base += al(8 * C);
-    double* q95r = reinterpret_cast<double*>(base); base += al(8 * C);
-    unsigned char* wqs = base;
+    double* q95r = reinterpret_cast<double*>(base);
     cudaMemsetAsync(isum, 0, 64 * C, s);
     cudaMemsetAsync(stretch, 0, 8 * C, s);
     const int tb = 256, gb = (b->t + tb - 1) / tb;
     k_quality_a<<<gb, tb, 0, s>>>(*b, tri, isum);
     k_quality_b<<<gb, tb, 0, s>>>(*b, tri, isum, qa, qr, per_aniso, per_area, stretch);
     UVA_CHECK_LAUNCH("uva_chart_quality");
-    // per-island quantiles: the island of triangle f is tri4[4 f + 3]
-    int rc = wquantile(b->t, qa.x, qa.w, b->tri4 + 3, 4, b->nc, 0.95, q95a, wqs, s);
-    if (rc == UVA_OK) rc = wquantile(b->t, qr.x, qr.w, b->tri4 + 3, 4, b->nc, 0.95, q95r, wqs, s);
-    if (rc != UVA_OK) return rc;
+    k_q_island<<<dim3(b->nc, 2), 256, 0, s>>>(b->tofs, qa.x, qa.w, q95a, qr.x, qr.w, q95r, 0.95);
     k_quality_out<<<(b->nc + tb - 1) / tb, tb, 0, s>>>(b->nc, isum, stretch, q95a, q95r, out);
     UVA_CHECK_LAUNCH("uva_chart_quality/out");
     return UVA_OK;
