@@ -22,9 +22,11 @@ using namespace uva;
 
 namespace {
 
+// FP64 issue bounds these kernels as much as memory: one reciprocal square
+// root each for |e1| and |n| replaces two square roots and five divisions.
 struct EnTri {
-    double e1[3], e2[3], n[3];
-    double l1, nn, x1, x2, y2, area;
+    double e1[3], e2[3], nh[3];     // edges, unit normal
+    double il, x2, y2, iy2, area;   // 1 / x1, the frame, 1 / y2
     double j00, j01, j10, j11;
     bool live;
 };
@@ -36,22 +38,25 @@ __device__ __forceinline__ EnTri en_tri(const double* P, const double* U, int v0
     const double* p2 = P + 3 * (v0 + tv.z);
 #pragma unroll
     for (int k = 0; k < 3; ++k) { t.e1[k] = p1[k] - p0[k]; t.e2[k] = p2[k] - p0[k]; }
-    t.n[0] = t.e1[1] * t.e2[2] - t.e1[2] * t.e2[1];
-    t.n[1] = t.e1[2] * t.e2[0] - t.e1[0] * t.e2[2];
-    t.n[2] = t.e1[0] * t.e2[1] - t.e1[1] * t.e2[0];
-    t.l1 = sqrt(t.e1[0] * t.e1[0] + t.e1[1] * t.e1[1] + t.e1[2] * t.e1[2]);
-    t.nn = sqrt(t.n[0] * t.n[0] + t.n[1] * t.n[1] + t.n[2] * t.n[2]);
-    const double il = 1.0 / fmax(t.l1, 1e-300);
-    t.x1 = t.l1;
-    t.x2 = (t.e1[0] * t.e2[0] + t.e1[1] * t.e2[1] + t.e1[2] * t.e2[2]) * il;
-    t.y2 = t.nn * il;   // e2 . (n/|n| x e1/|e1|) = |n| / |e1|
-    t.area = 0.5 * t.nn;
-    t.live = fabs(t.x1 * t.y2) >= 1e-300;
     const double2* UU = reinterpret_cast<const double2*>(U);
     const double2 u0 = UU[v0 + tv.x], u1 = UU[v0 + tv.y], u2 = UU[v0 + tv.z];
+    const double n0 = t.e1[1] * t.e2[2] - t.e1[2] * t.e2[1];
+    const double n1 = t.e1[2] * t.e2[0] - t.e1[0] * t.e2[2];
+    const double n2 = t.e1[0] * t.e2[1] - t.e1[1] * t.e2[0];
+    const double l1sq = t.e1[0] * t.e1[0] + t.e1[1] * t.e1[1] + t.e1[2] * t.e1[2];
+    const double nsq = n0 * n0 + n1 * n1 + n2 * n2;
+    const double inn = rsqrt(nsq), nn = nsq * inn;
+    t.il = rsqrt(l1sq);
+    t.x2 = (t.e1[0] * t.e2[0] + t.e1[1] * t.e2[1] + t.e1[2] * t.e2[2]) * t.il;
+    t.y2 = nn * t.il;   // e2 . (n/|n| x e1/|e1|) = |n| / |e1|
+    t.iy2 = l1sq * t.il * inn;
+    t.area = 0.5 * nn;
+    // x1 y2 = |n|; a zero normal or edge makes nn or il not a number
+    t.live = nn >= 1e-300 && t.il <= 1e300;
+    t.nh[0] = n0 * inn; t.nh[1] = n1 * inn; t.nh[2] = n2 * inn;
     if (t.live) {
-        t.j00 = (u1.x - u0.x) / t.x1; t.j10 = (u1.y - u0.y) / t.x1;
-        t.j01 = ((u2.x - u0.x) - t.j00 * t.x2) / t.y2; t.j11 = ((u2.y - u0.y) - t.j10 * t.x2) / t.y2;
+        t.j00 = (u1.x - u0.x) * t.il; t.j10 = (u1.y - u0.y) * t.il;
+        t.j01 = ((u2.x - u0.x) - t.j00 * t.x2) * t.iy2; t.j11 = ((u2.y - u0.y) - t.j10 * t.x2) * t.iy2;
     } else {
         t.j00 = t.j01 = t.j10 = t.j11 = 0.0;
     }
@@ -60,26 +65,26 @@ __device__ __forceinline__ EnTri en_tri(const double* P, const double* U, int v0
 
 // f(J) and dE/dJ per unit area; returns false for an inverted SD triangle.
 __device__ __forceinline__ bool en_f(const EnTri& t, int kind, double& f, double (&G)[4]) {
-    const double fro = t.j00 * t.j00 + t.j01 * t.j01 + t.j10 * t.j10 + t.j11 * t.j11;
     if (kind == 0) {
         const double qe = 0.5 * (t.j00 + t.j11), qh = 0.5 * (t.j10 - t.j01);
         const double rf = 0.5 * (t.j00 - t.j11), rg = 0.5 * (t.j10 + t.j01);
-        const double q = sqrt(qe * qe + qh * qh), r = sqrt(rf * rf + rg * rg);
+        const double q2 = qe * qe + qh * qh;
+        const double iq = q2 > 0.0 ? rsqrt(q2) : 0.0, q = q2 * iq, r = sqrt(rf * rf + rg * rg);
         f = (q + r - 1.0) * (q + r - 1.0) + (q - r - 1.0) * (q - r - 1.0);
-        double c = 0.0, s = 0.0;
-        if (q > 0.0) { c = qe / q; s = qh / q; }
+        const double c = qe * iq, s = qh * iq;
         G[0] = 2.0 * (t.j00 - c); G[1] = 2.0 * (t.j01 + s); G[2] = 2.0 * (t.j10 - s); G[3] = 2.0 * (t.j11 - c);
         return true;
     }
+    const double fro = t.j00 * t.j00 + t.j01 * t.j01 + t.j10 * t.j10 + t.j11 * t.j11;
     const double det = t.j00 * t.j11 - t.j01 * t.j10;
     if (!(det > 0.0)) {
         f = INFINITY;
         G[0] = G[1] = G[2] = G[3] = 0.0;
         return false;
     }
-    const double id2 = 1.0 / (det * det);
+    const double id = 1.0 / det, id2 = id * id;
     f = fro + fro * id2 - 4.0;
-    const double a = 2.0 * (1.0 + id2), b = -2.0 * fro * id2 / det;
+    const double a = 2.0 * (1.0 + id2), b = -2.0 * fro * id2 * id;
     G[0] = a * t.j00 + b * t.j11;
     G[1] = a * t.j01 - b * t.j10;
     G[2] = a * t.j10 - b * t.j01;
@@ -87,26 +92,20 @@ __device__ __forceinline__ bool en_f(const EnTri& t, int kind, double& f, double
     return true;
 }
 
-template <int K>
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// Triangles per thread of the forward pass: a thread sums a contiguous run
-// of triangles (islands are contiguous in triangle order), then the warp
-// folds runs of the same island, so an island's sum takes one FP64 atomic
-// per warp and island instead of one per triangle.
-constexpr int kFwdItems = 8;
-
-__global__ void k_energy_fwd(const uva_batch b, const double* P, const double* U, int kind, double* e_isl, double* e_tri) {
+// The forward pass gives a warp 32 * items consecutive triangles, lane by
+// lane. A lane sums its triangles of the same island (island ids do not
+// decrease along the triangles), then the warp folds lanes of equal islands,
+// so an island takes one FP64 atomic per warp. 5.1M triangles: 132 -> 82 us
+// (a thread's own run of eight strided its loads by 128 bytes).
+__global__ void k_energy_fwd(const uva_batch b, const double* P, const double* U, int kind, int items, double* e_isl,
+                             double* e_tri) {
     const int lane = threadIdx.x & 31;
-    const int64_t f0 = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * kFwdItems;
+    const int64_t f0 = (static_cast<int64_t>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31)) * items + lane;
     int isl = -1;
     double acc = 0.0;
-    for (int k = 0; k < kFwdItems; ++k) {
-        const int64_t f = f0 + k;
+#pragma unroll 2
+    for (int k = 0; k < items; ++k) {
+        const int64_t f = f0 + 32 * k;
         if (f >= b.t) break;
         const int4 tv = reinterpret_cast<const int4*>(b.tri4)[f];
         const EnTri t = en_tri(P, U, b.vofs[tv.w], tv);
@@ -117,15 +116,15 @@ __global__ void k_energy_fwd(const uva_batch b, const double* P, const double* U
             e = t.area * f_;
         }
         if (e_tri) e_tri[f] = e;
-        if (tv.w != isl) {   // a new island inside the run: flush the previous one
+        if (tv.w != isl) {   // a new island: flush the previous one
             if (isl >= 0 && acc != 0.0) atomicAdd(e_isl + isl, acc);
             isl = tv.w;
             acc = 0.0;
         }
         acc += e;
     }
-    // fold the lanes' last runs: island ids do not decrease along the lanes
-    // (idle lanes carry -1 and never match a live run)
+    // fold the lanes' last islands, which do not decrease along the lanes
+    // (idle lanes carry -1 and never match a live one)
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const double y = __shfl_down_sync(0xffffffffu, acc, o);
@@ -136,60 +135,85 @@ __global__ void k_energy_fwd(const uva_batch b, const double* P, const double* U
     if (isl >= 0 && (lane == 0 || prev != isl) && acc != 0.0) atomicAdd(e_isl + isl, acc);
 }
 
-__global__ void k_energy_bwd(const uva_batch b, const double* P, const double* U, int kind, const double* gscale,
-                             double* gU, double* gP) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= b.t) return;
-    const int4 tv = reinterpret_cast<const int4*>(b.tri4)[f];
-    const int v0 = b.vofs[tv.w];
-    const EnTri t = en_tri(P, U, v0, tv);
-    if (!t.live) return;
-    double f_, G[4];
-    if (!en_f(t, kind, f_, G)) return;
-    const double sc = gscale ? gscale[tv.w] : 1.0;
-    const double A = t.area * sc;
-    // dE/dJ = A G; J = D M^-1 with D = [du1 du2]: dE/dD = dE/dJ M^-T
-    const double g00 = A * G[0], g01 = A * G[1], g10 = A * G[2], g11 = A * G[3];
-    // M^-1 = [[1/x1, -x2/(x1 y2)], [0, 1/y2]]; dE/dD = g M^-T
-    const double ix1 = 1.0 / t.x1, iy2 = 1.0 / t.y2, m01 = -t.x2 / (t.x1 * t.y2);
-    const double d1x = g00 * ix1 + g01 * m01, d2x = g01 * iy2;
-    const double d1y = g10 * ix1 + g11 * m01, d2y = g11 * iy2;
-    double* gu = gU;
-    atomicAdd(gu + 2 * (v0 + tv.y), d1x); atomicAdd(gu + 2 * (v0 + tv.y) + 1, d1y);
-    atomicAdd(gu + 2 * (v0 + tv.z), d2x); atomicAdd(gu + 2 * (v0 + tv.z) + 1, d2y);
-    atomicAdd(gu + 2 * (v0 + tv.x), -(d1x + d2x)); atomicAdd(gu + 2 * (v0 + tv.x) + 1, -(d1y + d2y));
-    if (!gP) return;
-    // dE/dM = -J^T (A G) M^-T; M^-T = [[1/x1, 0], [m01, 1/y2]]
-    const double jg00 = t.j00 * g00 + t.j10 * g10, jg01 = t.j00 * g01 + t.j10 * g11;
-    const double jg10 = t.j01 * g00 + t.j11 * g10, jg11 = t.j01 * g01 + t.j11 * g11;
-    const double dM00 = -(jg00 * ix1 + jg01 * m01);    // d/dx1
-    const double dM01 = -(jg01 * iy2);                  // d/dx2 (row 0, col 1)
-    const double dM11 = -(jg11 * iy2);                  // d/dy2
-    (void)jg10;
-    const double dArea = sc * f_;
-    // x1 = |e1|; x2 = e1.e2/|e1|; y2 = |n|/|e1|; area = |n|/2
-    const double l1 = t.l1, nn = t.nn;
-    const double dot = t.e1[0] * t.e2[0] + t.e1[1] * t.e2[1] + t.e1[2] * t.e2[2];
-    double ge1[3], ge2[3];
-    const double nh[3] = {t.n[0] / fmax(nn, 1e-300), t.n[1] / fmax(nn, 1e-300), t.n[2] / fmax(nn, 1e-300)};
-    // d|n|/de1 = e2 x nh, d|n|/de2 = nh x e1
-    const double dn1[3] = {t.e2[1] * nh[2] - t.e2[2] * nh[1], t.e2[2] * nh[0] - t.e2[0] * nh[2], t.e2[0] * nh[1] - t.e2[1] * nh[0]};
-    const double dn2[3] = {nh[1] * t.e1[2] - nh[2] * t.e1[1], nh[2] * t.e1[0] - nh[0] * t.e1[2], nh[0] * t.e1[1] - nh[1] * t.e1[0]};
-    const double il = 1.0 / l1, il3 = il * il * il;
+// The global FP64 additions bound the backward pass: L2 takes some 230 G of
+// them a second, one operation per 32-byte sector that an instruction covers.
+// The corner gradients therefore pass through shared memory, and the lanes of
+// an addition take the components of a vertex side by side: one or two
+// operations per corner instead of five. 512 islands of 5.1M triangles, UV and
+// position gradients: 316 -> 192 us. (Summing a block's corners by vertex in a
+// shared hash table first took 281 us: its lookups cost more than they save.)
+constexpr int kBwdNT = 128;
+
+template <bool POS>
+__global__ void __launch_bounds__(kBwdNT) k_energy_bwd(const uva_batch b, const double* P, const double* U, int kind,
+                                                       const double* gscale, double* gU, double* gP) {
+    __shared__ double su[kBwdNT][6];
+    __shared__ double sp[POS ? kBwdNT : 1][9];
+    __shared__ int sv[kBwdNT][3];
+    const int f = blockIdx.x * kBwdNT + threadIdx.x;
+    int v[3] = {-1, -1, -1};
+    if (f < b.t) {
+        const int4 tv = reinterpret_cast<const int4*>(b.tri4)[f];
+        const int v0 = b.vofs[tv.w];
+        const EnTri t = en_tri(P, U, v0, tv);
+        double f_, G[4];
+        if (t.live && en_f(t, kind, f_, G)) {
+            v[0] = v0 + tv.x; v[1] = v0 + tv.y; v[2] = v0 + tv.z;
+            const double sc = gscale ? gscale[tv.w] : 1.0;
+            const double A = t.area * sc;
+            // dE/dJ = A G; J = D M^-1 with D = [du1 du2]: dE/dD = dE/dJ M^-T
+            // M^-1 = [[1/x1, -x2/(x1 y2)], [0, 1/y2]]
+            const double g00 = A * G[0], g01 = A * G[1], g10 = A * G[2], g11 = A * G[3];
+            const double m01 = -t.x2 * t.il * t.iy2;
+            const double d1x = g00 * t.il + g01 * m01, d2x = g01 * t.iy2;
+            const double d1y = g10 * t.il + g11 * m01, d2y = g11 * t.iy2;
+            double* o = su[threadIdx.x];
+            o[0] = -(d1x + d2x); o[1] = -(d1y + d2y);
+            o[2] = d1x; o[3] = d1y;
+            o[4] = d2x; o[5] = d2y;
+            if constexpr (POS) {
+                // dE/dM = -J^T (A G) M^-T
+                const double jg00 = t.j00 * g00 + t.j10 * g10, jg01 = t.j00 * g01 + t.j10 * g11;
+                const double jg11 = t.j01 * g01 + t.j11 * g11;
+                const double dM00 = -(jg00 * t.il + jg01 * m01);   // d/dx1
+                const double dM01 = -(jg01 * t.iy2);                // d/dx2 (row 0, col 1)
+                const double dM11 = -(jg11 * t.iy2);                // d/dy2
+                // x1 = |e1|, x2 = e1.e2 / |e1|, y2 = |n| / |e1|, area = |n| / 2;
+                // d|n|/de1 = e2 x nh, d|n|/de2 = nh x e1
+                const double il2 = t.il * t.il;
+                const double a1 = dM00 * t.il - il2 * (dM01 * t.x2 + dM11 * t.y2), a2 = dM01 * t.il;
+                const double an = dM11 * t.il + 0.5 * sc * f_;
+                const double dn1[3] = {t.e2[1] * t.nh[2] - t.e2[2] * t.nh[1], t.e2[2] * t.nh[0] - t.e2[0] * t.nh[2],
+                                       t.e2[0] * t.nh[1] - t.e2[1] * t.nh[0]};
+                const double dn2[3] = {t.nh[1] * t.e1[2] - t.nh[2] * t.e1[1], t.nh[2] * t.e1[0] - t.nh[0] * t.e1[2],
+                                       t.nh[0] * t.e1[1] - t.nh[1] * t.e1[0]};
+                double* w = sp[threadIdx.x];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const double dx1_de1 = t.e1[k] * il;
-        const double dx2_de1 = t.e2[k] * il - dot * t.e1[k] * il3, dx2_de2 = t.e1[k] * il;
-        const double dy2_de1 = dn1[k] * il - nn * t.e1[k] * il3, dy2_de2 = dn2[k] * il;
-        const double da_de1 = 0.5 * dn1[k], da_de2 = 0.5 * dn2[k];
-        ge1[k] = dM00 * dx1_de1 + dM01 * dx2_de1 + dM11 * dy2_de1 + dArea * da_de1;
-        ge2[k] = dM01 * dx2_de2 + dM11 * dy2_de2 + dArea * da_de2;
+                for (int k = 0; k < 3; ++k) {
+                    const double ge1 = a1 * t.e1[k] + a2 * t.e2[k] + an * dn1[k], ge2 = a2 * t.e1[k] + an * dn2[k];
+                    w[k] = -(ge1 + ge2);
+                    w[3 + k] = ge1;
+                    w[6 + k] = ge2;
+                }
+            }
+        }
     }
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        atomicAdd(gP + 3 * (v0 + tv.y) + k, ge1[k]);
-        atomicAdd(gP + 3 * (v0 + tv.z) + k, ge2[k]);
-        atomicAdd(gP + 3 * (v0 + tv.x) + k, -(ge1[k] + ge2[k]));
+    for (int k = 0; k < 3; ++k) sv[threadIdx.x][k] = v[k];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+        const int e = q * kBwdNT + threadIdx.x, c = e >> 1;
+        const int vv = (&sv[0][0])[c];
+        if (vv >= 0) atomicAdd(gU + 2 * static_cast<size_t>(vv) + (e & 1), (&su[0][0])[e]);
+    }
+    if constexpr (POS) {
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            const int e = q * kBwdNT + threadIdx.x, c = e / 3;
+            const int vv = (&sv[0][0])[c];
+            if (vv >= 0) atomicAdd(gP + 3 * static_cast<size_t>(vv) + (e - 3 * c), (&sp[0][0])[e]);
+        }
     }
 }
 
@@ -310,7 +334,9 @@ extern "C" int uva_energy_fwd(const uva_batch* b, const double* P, const double*
     if (!b || !P || !U || !e_isl || (kind != 0 && kind != 1)) { uva_set_error("uva_energy_fwd: bad arguments"); return UVA_E_ARG; }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaMemsetAsync(e_isl, 0, sizeof(double) * static_cast<size_t>(std::max(b->nc, 1)), s);
-    if (b->t > 0) k_energy_fwd<<<nb((b->t + kFwdItems - 1) / kFwdItems), 256, 0, s>>>(*b, P, U, kind, e_isl, e_tri);
+    // up to 8 triangles per thread once there are more than the GPU holds at a time
+    const int items = std::min(8, std::max(1, b->t / (148 * 1024)));
+    if (b->t > 0) k_energy_fwd<<<nb((b->t + items - 1) / items), 256, 0, s>>>(*b, P, U, kind, items, e_isl, e_tri);
     UVA_CHECK_LAUNCH("uva_energy_fwd");
     return UVA_OK;
 }
@@ -321,7 +347,9 @@ extern "C" int uva_energy_bwd(const uva_batch* b, const double* P, const double*
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaMemsetAsync(gU, 0, sizeof(double) * 2 * static_cast<size_t>(b->n), s);
     if (gP) cudaMemsetAsync(gP, 0, sizeof(double) * 3 * static_cast<size_t>(b->n), s);
-    if (b->t > 0) k_energy_bwd<<<nb(b->t), 256, 0, s>>>(*b, P, U, kind, gscale, gU, gP);
+    const int grid = (b->t + kBwdNT - 1) / kBwdNT;
+    if (b->t > 0 && gP) k_energy_bwd<true><<<grid, kBwdNT, 0, s>>>(*b, P, U, kind, gscale, gU, gP);
+    if (b->t > 0 && !gP) k_energy_bwd<false><<<grid, kBwdNT, 0, s>>>(*b, P, U, kind, gscale, gU, gP);
     UVA_CHECK_LAUNCH("uva_energy_bwd");
     return UVA_OK;
 }
