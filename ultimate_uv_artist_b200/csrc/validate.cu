@@ -76,48 +76,82 @@ __device__ __forceinline__ Tri load_tri(const UVT* UV, const int32_t* F, int t) 
     return r;
 }
 
-// Tolerant (engine/validate.py:57-91) and strict (:232-255) overlap of one
-// pair, evaluated together. bit0: tolerant, bit1: strict.
-__device__ int pair_overlap(const Tri& a, const Tri& b, double rel) {
-    bool same[3][3];
-    int shared = 0;
+// Corner coordinates of triangle t, packed by the classification (8 values of
+// stride: x0 y0 x1 y1 x2 y2): one or two sectors instead of three indexed pairs.
+template <typename UVT>
+__device__ __forceinline__ Tri packed_tri(const UVT* tri, int t) {
+    Tri r;
+    const UVT* c = tri + 8 * static_cast<size_t>(t);
+    if constexpr (sizeof(UVT) == 4) {
+        const float4 u = *reinterpret_cast<const float4*>(c);
+        const float2 v = *reinterpret_cast<const float2*>(c + 4);
+        r.x[0] = u.x; r.y[0] = u.y; r.x[1] = u.z; r.y[1] = u.w; r.x[2] = v.x; r.y[2] = v.y;
+    } else {
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        bool any = false;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            same[i][j] = a.x[i] == b.x[j] && a.y[i] == b.y[j];
-            any |= same[i][j];
+        for (int k = 0; k < 3; ++k) {
+            const double2 v = *reinterpret_cast<const double2*>(c + 2 * k);
+            r.x[k] = v.x; r.y[k] = v.y;
         }
-        shared += any ? 1 : 0;
     }
-    if (shared == 3) return 0;
-    int tol = 0, strict = 0;
+    return r;
+}
+
+template <typename UVT>
+__device__ __forceinline__ void pack_tri(UVT* tri, int t, const Tri& r) {
+    UVT* c = tri + 8 * static_cast<size_t>(t);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { c[2 * k] = static_cast<UVT>(r.x[k]); c[2 * k + 1] = static_cast<UVT>(r.y[k]); }
+}
+
+// Signs of 9 orientations: each edge i of t against the vertices j of o, bit
+// 3 i + j of pos / neg.
+__device__ __forceinline__ void edge_signs(const Tri& t, const Tri& o, unsigned& pos, unsigned& neg) {
+    pos = neg = 0;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        const int p0 = i, p1 = (i + 1) % 3;
+        const int n = (i + 1) % 3;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            const int q0 = j, q1 = (j + 1) % 3;
-            if (same[p0][q0] || same[p0][q1] || same[p1][q0] || same[p1][q1]) continue;
-            if (!tol && proper_cross(a.x[p0], a.y[p0], a.x[p1], a.y[p1], b.x[q0], b.y[q0], b.x[q1], b.y[q1], rel)) tol = 1;
+            const double d = orient(t.x[i], t.y[i], t.x[n], t.y[n], o.x[j], o.y[j]);
+            pos |= (d > 0.0 ? 1u : 0u) << (3 * i + j);
+            neg |= (d < 0.0 ? 1u : 0u) << (3 * i + j);
+        }
+    }
+}
+
+// Edge k of t keeps every vertex of the other triangle off its inner side.
+__device__ __forceinline__ bool separates(const Tri& t, unsigned pos, unsigned neg) {
+    const double area = orient(t.x[0], t.y[0], t.x[1], t.y[1], t.x[2], t.y[2]);
+    const unsigned in = area > 0.0 ? pos : (area < 0.0 ? neg : ~0u);
+    return !(in & 7u) || !(in & 56u) || !(in & 448u);
+}
+
+// Tolerant (engine/validate.py:57-91) and strict (:232-255) overlap of one
+// pair without a shared edge set of three vertices, in the reference's
+// operation order. `same`: bit 3 i + j, vertex i of a is vertex j of b.
+__device__ __noinline__ int pair_overlap_full(const Tri& a, const Tri& b, double rel, unsigned same) {
+    int tol = 0, strict = 0;
+    for (int i = 0; i < 3; ++i) {
+        const int p1 = (i + 1) % 3;
+        for (int j = 0; j < 3; ++j) {
+            const int q1 = (j + 1) % 3;
+            const unsigned ends = (1u << (3 * i + j)) | (1u << (3 * i + q1)) | (1u << (3 * p1 + j)) | (1u << (3 * p1 + q1));
+            if (same & ends) continue;   // edges with a shared end do not count
+            if (!tol && proper_cross(a.x[i], a.y[i], a.x[p1], a.y[p1], b.x[j], b.y[j], b.x[q1], b.y[q1], rel)) tol = 1;
             if (!strict) {
-                const double o1 = orient(a.x[p0], a.y[p0], a.x[p1], a.y[p1], b.x[q0], b.y[q0]);
-                const double o2 = orient(a.x[p0], a.y[p0], a.x[p1], a.y[p1], b.x[q1], b.y[q1]);
-                const double o3 = orient(b.x[q0], b.y[q0], b.x[q1], b.y[q1], a.x[p0], a.y[p0]);
-                const double o4 = orient(b.x[q0], b.y[q0], b.x[q1], b.y[q1], a.x[p1], a.y[p1]);
+                const double o1 = orient(a.x[i], a.y[i], a.x[p1], a.y[p1], b.x[j], b.y[j]);
+                const double o2 = orient(a.x[i], a.y[i], a.x[p1], a.y[p1], b.x[q1], b.y[q1]);
+                const double o3 = orient(b.x[j], b.y[j], b.x[q1], b.y[q1], a.x[i], a.y[i]);
+                const double o4 = orient(b.x[j], b.y[j], b.x[q1], b.y[q1], a.x[p1], a.y[p1]);
                 if (o1 * o2 < 0.0 && o3 * o4 < 0.0) strict = 1;
             }
         }
     }
-    if (!tol) {
-#pragma unroll
-        for (int i = 0; i < 3 && !tol; ++i) {
-            if (!(same[i][0] || same[i][1] || same[i][2]) &&
-                strict_inside(a.x[i], a.y[i], b.x[0], b.y[0], b.x[1], b.y[1], b.x[2], b.y[2], rel)) tol = 1;
-            if (!tol && !(same[0][i] || same[1][i] || same[2][i]) &&
-                strict_inside(b.x[i], b.y[i], a.x[0], a.y[0], a.x[1], a.y[1], a.x[2], a.y[2], rel)) tol = 1;
-        }
+    for (int i = 0; i < 3 && !tol; ++i) {
+        if (!(same & (7u << (3 * i))) &&
+            strict_inside(a.x[i], a.y[i], b.x[0], b.y[0], b.x[1], b.y[1], b.x[2], b.y[2], rel)) tol = 1;
+        if (!tol && !(same & (73u << i)) &&
+            strict_inside(b.x[i], b.y[i], a.x[0], a.y[0], a.x[1], a.y[1], a.x[2], a.y[2], rel)) tol = 1;
     }
     if (!tol) {
         const double cx = (a.x[0] + a.x[1] + a.x[2]) / 3.0, cy = (a.y[0] + a.y[1] + a.y[2]) / 3.0;
@@ -128,6 +162,47 @@ __device__ int pair_overlap(const Tri& a, const Tri& b, double rel) {
         if (strict_inside(cx, cy, a.x[0], a.y[0], a.x[1], a.y[1], a.x[2], a.y[2], rel)) tol = 1;
     }
     return tol | (strict << 1);
+}
+
+// The same, bit0: tolerant, bit1: strict, with a filter in front. Every
+// predicate combines 18 orientations (each edge of one triangle against the
+// vertices of the other), and asks for signs before sizes:
+//  * a crossing, tolerant or strict: opposite signs of both pairs of an edge
+//    pair without a shared end;
+//  * an inside vertex: one sign against all three edges;
+//  * an inside centroid: not possible by the tolerance (at least 2.4e-7 of a
+//    length) when an edge has none of the other's vertices on its inner side:
+//    an orientation is affine, and round-off on coordinates below 1e6 is under
+//    1e-9 of a length. `big`: a larger coordinate, or no relative tolerance.
+// Most candidates (neighbours across an edge or a vertex) end here with 20
+// orientations; the others evaluate everything.
+__device__ __forceinline__ int pair_overlap(const Tri& a, const Tri& b, double rel, bool big) {
+    unsigned same = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) same |= (a.x[i] == b.x[j] && a.y[i] == b.y[j] ? 1u : 0u) << (3 * i + j);
+    if ((same & 7u) && (same & 56u) && (same & 448u)) return 0;   // three shared vertices
+    unsigned pa, na, pb, nb;
+    edge_signs(a, b, pa, na);
+    edge_signs(b, a, pb, nb);
+    bool maybe = big || !separates(a, pa, na) || !separates(b, pb, nb);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int p1 = (i + 1) % 3;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int q1 = (j + 1) % 3;
+            const unsigned ends = (1u << (3 * i + j)) | (1u << (3 * i + q1)) | (1u << (3 * p1 + j)) | (1u << (3 * p1 + q1));
+            const unsigned a1 = 1u << (3 * i + j), a2 = 1u << (3 * i + q1), b1 = 1u << (3 * j + i), b2 = 1u << (3 * j + p1);
+            maybe |= !(same & ends) && (((pa & a1) && (na & a2)) || ((na & a1) && (pa & a2))) &&
+                     (((pb & b1) && (nb & b2)) || ((nb & b1) && (pb & b2)));
+        }
+        const unsigned col = 73u << i;   // vertex i against the three edges
+        maybe |= !(same & (7u << (3 * i))) && ((pb & col) == col || (nb & col) == col);
+        maybe |= !(same & col) && ((pa & col) == col || (na & col) == col);
+    }
+    return maybe ? pair_overlap_full(a, b, rel, same) : 0;
 }
 
 // ------------------------------------------------------------------ helpers
@@ -175,11 +250,12 @@ __global__ void k_v_area3(int m, const double* V, const int32_t* F, double* a3, 
 
 // engine/validate.py:149-172: signed area, sliver, has3d, skip; cell boxes.
 __global__ void k_v_classify(int m, const float* UV, const int32_t* F, const double* a3, const double* amax, int G,
-                             double* sa_out, uint8_t* tflags, int4* cbox, unsigned long long* counts) {
+                             float* tri, double* sa_out, uint8_t* tflags, int4* cbox, unsigned long long* counts) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     bool deg = false, sl = false;
     if (t < m) {
         const Tri r = load_tri(UV, F, t);
+        pack_tri(tri, t, r);
         const double sa = 0.5 * ((r.x[1] - r.x[0]) * (r.y[2] - r.y[0]) - (r.x[2] - r.x[0]) * (r.y[1] - r.y[0]));
         const double e0 = sqrt((r.x[1] - r.x[0]) * (r.x[1] - r.x[0]) + (r.y[1] - r.y[0]) * (r.y[1] - r.y[0]));
         const double e1 = sqrt((r.x[2] - r.x[1]) * (r.x[2] - r.x[1]) + (r.y[2] - r.y[1]) * (r.y[2] - r.y[1]));
@@ -362,14 +438,34 @@ __global__ void k_labels(int m, const int32_t* froot, const int32_t* rank, int32
     if (t < m) labels[t] = rank[froot[t]];
 }
 
+// Sums of the positive and negative areas and the triangles per island, folded
+// over the runs of equal labels along a warp (labels may come in any order)
+// before the atomics.
 __global__ void k_orient_sums(int m, const double* sa, const int32_t* labels, double* pos, double* neg, int32_t* cnt) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= m) return;
-    const double s = sa[t];
-    const int l = labels[t];
-    if (s > 0.0) atomicAdd(pos + l, s);
-    else if (s < 0.0) atomicAdd(neg + l, -s);
-    atomicAdd(cnt + l, 1);
+    const int lane = threadIdx.x & 31;
+    double p = 0.0, q = 0.0;
+    int l = -1;
+    if (t < m) {
+        const double s = sa[t];
+        if (s > 0.0) p = s;
+        else if (s < 0.0) q = -s;
+        l = labels[t];
+    }
+    const int prev = __shfl_up_sync(0xffffffffu, l, 1);
+    const bool head = lane == 0 || prev != l;
+    const unsigned heads = __ballot_sync(0xffffffffu, head);
+    const unsigned above = lane == 31 ? 0u : heads & (0xfffffffeu << lane);
+    const int end = above ? __ffs(above) - 1 : 32;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double yp = __shfl_down_sync(0xffffffffu, p, o), yq = __shfl_down_sync(0xffffffffu, q, o);
+        if (lane + o < end) { p += yp; q += yq; }
+    }
+    if (l < 0 || !head) return;
+    if (p != 0.0) atomicAdd(pos + l, p);
+    if (q != 0.0) atomicAdd(neg + l, q);
+    atomicAdd(cnt + l, end - lane);
 }
 
 // dom = pos >= neg. Sums of k non-negative terms in any order are within
@@ -441,9 +537,8 @@ __global__ void k_bin_fill(int m, const int4* cbox, int G, const int32_t* cofs, 
 }
 
 template <typename UVT>
-__device__ __forceinline__ void test_pair(int s, int t, const UVT* UV, const int32_t* F, double rel, uint8_t* tflags,
-                                          bool& counted) {
-    const Tri a = load_tri(UV, F, s), b = load_tri(UV, F, t);
+__device__ __forceinline__ bool test_pair(int s, int t, const UVT* tri, double rel, uint8_t* tflags) {
+    const Tri a = packed_tri(tri, s), b = packed_tri(tri, t);
     double alx = a.x[0], ahx = a.x[0], aly = a.y[0], ahy = a.y[0];
     double blx = b.x[0], bhx = b.x[0], bly = b.y[0], bhy = b.y[0];
 #pragma unroll
@@ -451,43 +546,81 @@ __device__ __forceinline__ void test_pair(int s, int t, const UVT* UV, const int
         alx = fmin(alx, a.x[k]); ahx = fmax(ahx, a.x[k]); aly = fmin(aly, a.y[k]); ahy = fmax(ahy, a.y[k]);
         blx = fmin(blx, b.x[k]); bhx = fmax(bhx, b.x[k]); bly = fmin(bly, b.y[k]); bhy = fmax(bhy, b.y[k]);
     }
-    if (alx > bhx || blx > ahx || aly > bhy || bly > ahy) return;   // real boxes disjoint: no overlap possible
-    counted = true;
-    const int r = pair_overlap(a, b, rel);
+    if (alx > bhx || blx > ahx || aly > bhy || bly > ahy) return false;   // real boxes disjoint: no overlap possible
+    // coordinates on which the centroid shortcut does not hold
+    const bool big = !(rel > 0.0) || !(fmin(fmin(alx, blx), fmin(aly, bly)) > -1e6 && fmax(fmax(ahx, bhx), fmax(ahy, bhy)) < 1e6);
+    const int r = pair_overlap(a, b, rel, big);
     if (r) {
         const uint8_t bits = static_cast<uint8_t>(((r & 1) ? 16 : 0) | ((r & 2) ? 32 : 0));
         atomicOr(reinterpret_cast<unsigned int*>(tflags + (s & ~3)), static_cast<unsigned int>(bits) << (8 * (s & 3)));
         atomicOr(reinterpret_cast<unsigned int*>(tflags + (t & ~3)), static_cast<unsigned int>(bits) << (8 * (t & 3)));
     }
+    return true;
 }
 
-// One thread per (cell, item): pairs with the later items of the cell, each
-// pair once (in the first cell both cell boxes share, engine/validate.py:130).
-// Only cells of rows [band_lo, band_hi): a shard's band of the atlas.
+// Pairs of the items of a cell, each pair once (in the first cell both cell
+// boxes share, engine/validate.py:130). A lane walks the later items of its
+// item's cell; the pairs that share the cell go to the warp's queue, and the
+// predicates run on 32 of them at a time. Only cells of rows
+// [band_lo, band_hi): a shard's band of the atlas. 1M triangles, 7.3M
+// candidate pairs: 0.66 ms; 3.08 ms with a lane testing its own pairs as it met
+// them, up to 72 orientations and 20 square roots each (and 1.4 ms at one
+// block per SM, which 138 registers allowed; three blocks spill a little).
+constexpr int kPairNT = 256;
+
 template <typename UVT>
-__global__ void k_pairs_items(const int32_t* nitems, const int32_t* items, const int32_t* item_cell, const int32_t* cofs,
-                              const int4* cbox, int G, const UVT* UV, const int32_t* F, double rel, uint8_t* tflags,
-                              unsigned long long* counts, int band_lo, int band_hi) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kPairNT, 3) k_pairs_items(const int32_t* nitems, const int32_t* items,
+                                                         const int32_t* item_cell, const int32_t* cofs,
+                                                         const int4* cbox, int G, const UVT* tri, double rel,
+                                                         uint8_t* tflags, unsigned long long* counts, int band_lo,
+                                                         int band_hi) {
+    __shared__ int2 queue[kPairNT / 32][64];
+    const int lane = threadIdx.x & 31;
+    int2* qu = queue[threadIdx.x >> 5];
+    const int n = *nitems;
     unsigned long long npairs = 0;
-    if (p < *nitems && item_cell[p] / G >= band_lo && item_cell[p] / G < band_hi) {
-        const int cell = item_cell[p];
-        const int cx = cell % G, cy = cell / G;
-        const int end = cofs[cell + 1];
-        const int s = items[p];
-        const int4 bs = cbox[s];
-        for (int q = p + 1; q < end; ++q) {
-            const int t = items[q];
-            const int4 bt = cbox[t];
-            if (max(bs.x, bt.x) != cx || max(bs.z, bt.z) != cy) continue;
-            if (bs.x > bt.y || bt.x > bs.y || bs.z > bt.w || bt.z > bs.w) continue;
-            bool counted = false;
-            test_pair(s, t, UV, F, rel, tflags, counted);
-            npairs += counted ? 1 : 0;
+    int nq = 0;   // queued pairs (the same on every lane)
+    for (int base = blockIdx.x * kPairNT + (threadIdx.x & ~31); base < n; base += gridDim.x * kPairNT) {
+        const int p = base + lane;
+        int cx = 0, cy = 0, s = 0, q = 0, end = 0;
+        int4 bs = make_int4(0, 0, 0, 0);
+        if (p < n) {
+            const int cell = item_cell[p];
+            cx = cell % G; cy = cell / G;
+            if (cy >= band_lo && cy < band_hi) {
+                q = p + 1;
+                end = cofs[cell + 1];
+                s = items[p];
+                bs = cbox[s];
+            }
+        }
+        while (__any_sync(0xffffffffu, q < end)) {
+            bool cand = false;
+            int t = 0;
+            if (q < end) {
+                t = items[q++];
+                const int4 bt = cbox[t];
+                cand = max(bs.x, bt.x) == cx && max(bs.z, bt.z) == cy && bs.x <= bt.y && bt.x <= bs.y &&
+                       bs.z <= bt.w && bt.z <= bs.w;
+            }
+            const unsigned mask = __ballot_sync(0xffffffffu, cand);
+            if (cand) qu[nq + __popc(mask & ((1u << lane) - 1u))] = make_int2(s, t);
+            nq += __popc(mask);
+            __syncwarp();
+            if (nq >= 32) {
+                nq -= 32;
+                const int2 pr = qu[nq + lane];
+                npairs += test_pair(pr.x, pr.y, tri, rel, tflags) ? 1 : 0;
+                __syncwarp();
+            }
         }
     }
+    if (lane < nq) {
+        const int2 pr = qu[lane];
+        npairs += test_pair(pr.x, pr.y, tri, rel, tflags) ? 1 : 0;
+    }
     for (int o = 16; o > 0; o >>= 1) npairs += __shfl_xor_sync(0xffffffffu, npairs, o);
-    if ((threadIdx.x & 31) == 0 && npairs) atomicAdd(counts + UVA_VC_PAIRS, npairs);
+    if (lane == 0 && npairs) atomicAdd(counts + UVA_VC_PAIRS, npairs);
 }
 
 // item -> cell map for k_pairs (cells own contiguous item ranges)
@@ -502,7 +635,7 @@ __global__ void k_item_cells(int ncells, const int32_t* cofs, int32_t* item_cell
 // band holding the row of its first shared cell, as on the binned path.
 template <typename UVT>
 __global__ void k_pairs_big(int m, const int32_t* big, const int32_t* nbig, const int4* cbox, const uint8_t* skipf,
-                            const UVT* UV, const int32_t* F, double rel, uint8_t* tflags, unsigned long long* counts,
+                            const UVT* tri, double rel, uint8_t* tflags, unsigned long long* counts,
                             int band_lo, int band_hi) {
     const int nb = *nbig;
     unsigned long long npairs = 0;
@@ -517,9 +650,7 @@ __global__ void k_pairs_big(int m, const int32_t* big, const int32_t* nbig, cons
             if (bs.x > bt.y || bt.x > bs.y || bs.z > bt.w || bt.z > bs.w) continue;
             const int cy = max(bs.z, bt.z);
             if (cy < band_lo || cy >= band_hi) continue;
-            bool counted = false;
-            test_pair(s, t, UV, F, rel, tflags, counted);
-            npairs += counted ? 1 : 0;
+            npairs += test_pair(s, t, tri, rel, tflags) ? 1 : 0;
         }
     }
     for (int o = 16; o > 0; o >>= 1) npairs += __shfl_xor_sync(0xffffffffu, npairs, o);
@@ -587,10 +718,12 @@ __global__ void k_store_pairs_meta(const int32_t* nbig, const int32_t* namb, uns
 }
 
 // engine/validate.py:221-226: FP64 normalised chart UVs, skip |sa| <= 1e-14.
-__global__ void k_chart_classify(int m, const double* U, const int32_t* F, int G, uint8_t* tflags, int4* cbox) {
+__global__ void k_chart_classify(int m, const double* U, const int32_t* F, int G, double* tri, uint8_t* tflags,
+                                 int4* cbox) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= m) return;
     const Tri r = load_tri(U, F, t);
+    pack_tri(tri, t, r);
     const double sa = 0.5 * ((r.x[1] - r.x[0]) * (r.y[2] - r.y[0]) - (r.x[2] - r.x[0]) * (r.y[1] - r.y[0]));
     const bool skip = fabs(sa) <= 1e-14;
     tflags[t] = skip ? 4 : 0;
@@ -642,9 +775,10 @@ Layout layout(int64_t n, int64_t m, int64_t G) {
         4 * (m + 1),               // 19 island overlap flag
         4 * nb,                    // 20 scan block sums
         64,                        // 21 small ints (totals, counters)
+        64 * m,                    // 22 packed corners (8 floats or doubles per triangle)
     };
     size_t o = 0;
-    for (int i = 0; i < 22; ++i) {
+    for (int i = 0; i < 23; ++i) {
         L.off[i] = o;
         o += (static_cast<size_t>(sizes[i]) + 255) & ~static_cast<size_t>(255);
     }
@@ -720,7 +854,8 @@ extern "C" int uva_validate(const uva_val_desc* d, void* stream) {
     if (m == 0) { UVA_CHECK_LAUNCH("uva_validate"); return UVA_OK; }
     cudaMemsetAsync(amax, 0, sizeof(double), s);
     k_v_area3<<<blocks(m), 256, 0, s>>>(m, d->V, d->F, a3, amax);
-    k_v_classify<<<blocks(m), 256, 0, s>>>(m, d->UV, d->F, a3, amax, G, d->sa, d->tflags, cbox, counts);
+    float* tri = reinterpret_cast<float*>(R(22));
+    k_v_classify<<<blocks(m), 256, 0, s>>>(m, d->UV, d->F, a3, amax, G, tri, d->sa, d->tflags, cbox, counts);
     UVA_CHECK_LAUNCH("uva_validate/classify");
     // islands
     cudaMemsetAsync(table, 0xff, static_cast<size_t>(hmask + 1) * 4, s);
@@ -749,15 +884,13 @@ extern "C" int uva_validate(const uva_val_desc* d, void* stream) {
     k_bin_fill<<<blocks(m), 256, 0, s>>>(m, cbox, G, cofs, cursor, items);
     k_item_cells<<<blocks(ncell), 256, 0, s>>>(ncell, cofs, item_cell);
     UVA_CHECK_LAUNCH("uva_validate/binning");
-    // the number of items is bounded by kMaxCells * m; threads beyond the
-    // actual count read cofs[ncell] as the end and do nothing
     const int nsh = std::max(1, d->nshards), sh = nsh > 1 ? d->shard : 0;
     const int band_lo = static_cast<int>(static_cast<int64_t>(G) * sh / nsh);
     const int band_hi = static_cast<int>(static_cast<int64_t>(G) * (sh + 1) / nsh);
-    k_pairs_items<float><<<blocks(kMaxCells * m), 256, 0, s>>>(nitems, items, item_cell, cofs, cbox, G, d->UV, d->F,
-                                                                d->rel, d->tflags, counts, band_lo, band_hi);
-    k_pairs_big<float><<<148, 256, 0, s>>>(m, big, nbig, cbox, d->tflags, d->UV, d->F, d->rel, d->tflags, counts,
-                                           band_lo, band_hi);
+    k_pairs_items<float><<<std::min(blocks(m), 148 * 8), kPairNT, 0, s>>>(nitems, items, item_cell, cofs, cbox, G, tri,
+                                                                          d->rel, d->tflags, counts, band_lo, band_hi);
+    k_pairs_big<float><<<148, 256, 0, s>>>(m, big, nbig, cbox, d->tflags, tri, d->rel, d->tflags, counts, band_lo,
+                                           band_hi);
     UVA_CHECK_LAUNCH("uva_validate/pairs");
     cudaMemsetAsync(isl_ov, 0, 4 * static_cast<size_t>(m + 1), s);
     k_final<<<blocks(m), 256, 0, s>>>(m, d->sa, d->labels, dom, d->tflags, isl_ov, counts);
@@ -822,14 +955,15 @@ extern "C" int uva_chart_overlaps(const double* U, const int32_t* F, int32_t n, 
     cudaMemsetAsync(smalls, 0, 64, s);
     cudaMemsetAsync(ccount, 0, 4 * static_cast<size_t>(ncell + 1), s);
     cudaMemsetAsync(cursor, 0, 4 * static_cast<size_t>(ncell), s);
-    k_chart_classify<<<blocks(m), 256, 0, s>>>(m, U, F, G, tflags, cbox);
+    double* tri = reinterpret_cast<double*>(R(22));
+    k_chart_classify<<<blocks(m), 256, 0, s>>>(m, U, F, G, tri, tflags, cbox);
     k_bin_count<<<blocks(m), 256, 0, s>>>(m, cbox, G, ccount, big, smalls + 1);
     scan(ccount, cofs, sums, smalls + 3, ncell + 1, s);
     k_bin_fill<<<blocks(m), 256, 0, s>>>(m, cbox, G, cofs, cursor, items);
     k_item_cells<<<blocks(ncell), 256, 0, s>>>(ncell, cofs, item_cell);
-    k_pairs_items<double><<<blocks(kMaxCells * m), 256, 0, s>>>(smalls + 3, items, item_cell, cofs, cbox, G, U, F, 1e-6,
-                                                                 tflags, counts, 0, G);
-    k_pairs_big<double><<<148, 256, 0, s>>>(m, big, smalls + 1, cbox, tflags, U, F, 1e-6, tflags, counts, 0, G);
+    k_pairs_items<double><<<std::min(blocks(m), 148 * 8), kPairNT, 0, s>>>(smalls + 3, items, item_cell, cofs, cbox, G,
+                                                                           tri, 1e-6, tflags, counts, 0, G);
+    k_pairs_big<double><<<148, 256, 0, s>>>(m, big, smalls + 1, cbox, tflags, tri, 1e-6, tflags, counts, 0, G);
     UVA_CHECK_LAUNCH("uva_chart_overlaps");
     return UVA_OK;
 }
