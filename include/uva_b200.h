@@ -177,6 +177,10 @@ int uva_concat_tris32(int32_t nc, const void* const* T, const int8_t* tdt, const
  * parallel (positions that are float32 upload as they are).               */
 int uva_concat_rows32(int32_t nc, const void* const* src, const int64_t* ofs, int32_t width, float* out,
                       int32_t nthreads);
+/* Host elements into a (page-locked) buffer of the same type, or float64 ->
+ * float32, int64 -> int32, over up to 8 threads. Codes: 0 float32, 1 float64,
+ * 2 int32, 3 int64. */
+int uva_stage(const void* src, int32_t src_code, void* dst, int32_t dst_code, int64_t count);
 int uva_dplan_scratch_bytes(int64_t n, int64_t t, int64_t nslices, int64_t* bytes);
 int uva_dplan_build(const uva_dplan* d, void* stream);
 int uva_dplan_slots(const uva_dplan* d, int32_t* slot_col, int32_t* slot_edge, float* slot_c, void* stream);

@@ -14,7 +14,9 @@
 #include <cstring>
 #include <memory>
 #include <numeric>
+#include <system_error>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/uva_b200.h"
@@ -621,6 +623,62 @@ extern "C" int uva_concat_rows32(int32_t nc, const void* const* src, const int64
     nt = std::max(1, std::min(nt, std::max(nc, 1)));
     std::vector<std::thread> pool;
     for (int32_t k = 1; k < nt; ++k) pool.emplace_back(worker);
+    worker();
+    for (auto& th : pool) th.join();
+    return UVA_OK;
+}
+
+// Elements of one host array into another (a page-locked staging buffer) in the
+// destination's type, in ranges over up to 8 threads: 0 float32, 1 float64,
+// 2 int32, 3 int64. float64 -> float32 rounds to nearest and int64 -> int32
+// keeps the low bits, as numpy's astype does.
+namespace {
+
+template <typename S, typename D>
+void cast_range(const void* src, void* dst, int64_t lo, int64_t hi) {
+    const S* s = static_cast<const S*>(src);
+    D* d = static_cast<D*>(dst);
+    if (std::is_same<S, D>::value) {
+        std::memcpy(d + lo, s + lo, sizeof(D) * static_cast<size_t>(hi - lo));
+    } else {
+        for (int64_t k = lo; k < hi; ++k) d[k] = static_cast<D>(s[k]);
+    }
+}
+
+}  // namespace
+
+extern "C" int uva_stage(const void* src, int32_t src_code, void* dst, int32_t dst_code, int64_t count) {
+    using Fn = void (*)(const void*, void*, int64_t, int64_t);
+    Fn fn = nullptr;
+    if (src_code == dst_code) {
+        static const Fn same[4] = {cast_range<float, float>, cast_range<double, double>, cast_range<int32_t, int32_t>,
+                                   cast_range<int64_t, int64_t>};
+        if (src_code >= 0 && src_code < 4) fn = same[src_code];
+    } else if (src_code == 1 && dst_code == 0) {
+        fn = cast_range<double, float>;
+    } else if (src_code == 3 && dst_code == 2) {
+        fn = cast_range<int64_t, int32_t>;
+    }
+    if (!fn || count < 0 || (count > 0 && (!src || !dst))) {
+        uva_set_error("uva_stage: bad arguments");
+        return UVA_E_ARG;
+    }
+    constexpr int64_t kRange = 1 << 18;   // elements; below two ranges a thread costs more than it saves
+    const int64_t ranges = (count + kRange - 1) / kRange;
+    std::atomic<int64_t> next{0};
+    auto worker = [&]() {
+        for (;;) {
+            const int64_t r = next.fetch_add(1);
+            if (r >= ranges) break;
+            fn(src, dst, r * kRange, std::min(count, (r + 1) * kRange));
+        }
+    };
+    const int64_t nt = std::min<int64_t>({8, ranges, std::max<int64_t>(1, std::thread::hardware_concurrency())});
+    std::vector<std::thread> pool;
+    try {
+        for (int64_t k = 1; k < nt; ++k) pool.emplace_back(worker);
+    } catch (const std::system_error&) {   // no more threads: the ones that started and this one do it
+    }
     worker();
     for (auto& th : pool) th.join();
     return UVA_OK;

@@ -78,6 +78,35 @@ def to_host(t):
     return out
 
 
+_STAGE_CODE = {np.dtype(np.float32): 0, np.dtype(np.float64): 1, np.dtype(np.int32): 2, np.dtype(np.int64): 3}
+_STAGE_MIN = 1 << 15   # elements: smaller arrays go through one pageable copy
+
+
+def upload(a, dtype, dev):
+    """Array-like ``a`` on device ``dev`` as a contiguous tensor of ``dtype``
+    (float32, float64, int32 or int64). Large arrays are staged into
+    page-locked memory by the host cores, narrowed to the target type on the
+    way, and copied asynchronously; float32 values for a float64 target travel
+    as float32 and are widened on the device (exact). The staging tensor comes
+    from torch's caching host allocator, which reuses its memory only after the
+    copy has run. A pageable copy of 66 MB (1.8M triangles) took 4.6 ms and its
+    conversions as much again."""
+    a = np.asarray(a)
+    dtype = np.dtype(dtype)
+    src = np.dtype(np.float32) if a.dtype == np.float32 and dtype == np.float64 else dtype
+    pair = (a.dtype, src)
+    staged = a.size >= _STAGE_MIN and (a.dtype == src or pair in ((np.dtype(np.float64), np.dtype(np.float32)),
+                                                                  (np.dtype(np.int64), np.dtype(np.int32))))
+    if not staged or src not in _STAGE_CODE:
+        return torch.from_numpy(np.ascontiguousarray(a, dtype)).to(dev)
+    a = np.ascontiguousarray(a)
+    t = torch.empty(a.shape, dtype=_TORCH_OF[src], pin_memory=True)
+    check(_lib.lib().uva_stage(ptr(a), _STAGE_CODE[a.dtype], C.c_void_p(t.data_ptr()), _STAGE_CODE[src], a.size),
+          "uva_stage")
+    out = t.to(dev, non_blocking=True)
+    return out if src == dtype else out.to(_TORCH_OF[dtype])
+
+
 class Plan:
     """Host topology plan (wraps uva_plan_create / uva_plan_export)."""
 

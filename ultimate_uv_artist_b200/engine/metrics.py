@@ -15,7 +15,7 @@ import numpy as np
 import torch
 
 from .. import _lib, meshops
-from ..device import require_cuda, to_host
+from ..device import require_cuda, to_host, upload
 
 vp = C.c_void_p
 
@@ -66,8 +66,8 @@ def _raster_counts(uv, faces, res, counts):
 def _raster_counts_device(uv, faces, res):
     L = _sig()
     dev = require_cuda()
-    U = torch.from_numpy(np.ascontiguousarray(uv, np.float64)).to(dev)
-    F = torch.from_numpy(np.ascontiguousarray(faces, np.int32).reshape(-1, 3)).to(dev)
+    U = upload(uv, np.float64, dev)
+    F = upload(faces, np.int32, dev).reshape(-1, 3)
     m = int(F.shape[0])
     out = torch.empty((res, res), dtype=torch.uint8, device=dev)
     stats = torch.zeros(2, dtype=torch.int64, device=dev)
@@ -93,13 +93,13 @@ def uv_islands(faces, n_vertices, uv=None, vertices=None):
     partition equals the reference's."""
     L = _sig()
     dev = require_cuda()
-    F = torch.from_numpy(np.ascontiguousarray(faces, np.int32).reshape(-1, 3)).to(dev)
+    F = upload(faces, np.int32, dev).reshape(-1, 3)
     m = int(F.shape[0])
     n = int(n_vertices)
     weld = uv is not None and vertices is not None
     if weld:
-        V = torch.from_numpy(np.ascontiguousarray(vertices, np.float64).reshape(-1, 3)).to(dev)
-        UV = torch.from_numpy(np.ascontiguousarray(uv, np.float32).reshape(-1, 2)).to(dev)
+        V = upload(vertices, np.float64, dev).reshape(-1, 3)
+        UV = upload(uv, np.float32, dev).reshape(-1, 2)
         n = int(V.shape[0])
     else:
         V = UV = None
@@ -122,8 +122,8 @@ def _wquantile(x, w, q):
     w = np.asarray(w, np.float64)
     if len(x) == 0:
         return float("nan")
-    X = torch.from_numpy(np.ascontiguousarray(x)).to(dev)
-    W = torch.from_numpy(np.ascontiguousarray(w)).to(dev)
+    X = upload(x, np.float64, dev)
+    W = upload(w, np.float64, dev)
     out = torch.empty(1, dtype=torch.float64, device=dev)
     nb = C.c_int64()
     _lib.check(L.uva_wquantile_scratch_bytes(1, C.byref(nb)), "uva_wquantile_scratch_bytes")
@@ -151,10 +151,10 @@ def _distortion(V, F, UV, islands, n_islands, per_tri="host", keep_per_tri=False
     not written (the kernel keeps it in its scratch)."""
     L = _sig()
     dev = require_cuda()
-    Vt = torch.from_numpy(np.ascontiguousarray(V, np.float64).reshape(-1, 3)).to(dev)
-    Ft = torch.from_numpy(np.ascontiguousarray(F, np.int32).reshape(-1, 3)).to(dev)
-    Ut = torch.from_numpy(np.ascontiguousarray(UV, np.float64).reshape(-1, 2)).to(dev)
-    It = torch.from_numpy(np.ascontiguousarray(islands, np.int32)).to(dev) if islands is not None else None
+    Vt = upload(V, np.float64, dev).reshape(-1, 3)
+    Ft = upload(F, np.int32, dev).reshape(-1, 3)
+    Ut = upload(UV, np.float64, dev).reshape(-1, 2)
+    It = upload(islands, np.int32, dev) if islands is not None else None
     m = int(Ft.shape[0])
     out = torch.zeros(32, dtype=torch.float64, device=dev)
     want = keep_per_tri or per_tri is not None
@@ -287,9 +287,9 @@ def _raster_labels(uv, faces, lab_of_face, res, img):
     fills ``img`` (res x res int32) in place."""
     L = _sig()
     dev = require_cuda()
-    UV = torch.from_numpy(np.ascontiguousarray(uv, np.float64)).to(dev)
-    F = torch.from_numpy(np.ascontiguousarray(faces, np.int32).reshape(-1, 3)).to(dev)
-    lab = torch.from_numpy(np.ascontiguousarray(lab_of_face, np.int32)).to(dev)
+    UV = upload(uv, np.float64, dev)
+    F = upload(faces, np.int32, dev).reshape(-1, 3)
+    lab = upload(lab_of_face, np.int32, dev)
     out, _ = _gutter_raw(UV, F, lab, int(res), 1)
     res_img = to_host(out)
     np.copyto(img, np.where(res_img >= 0, res_img, img))
@@ -334,9 +334,9 @@ def min_gutter(uv, faces, islands, res=4096):
     """Smallest texel gap between two different islands (engine/metrics.py:348-373).
     Returns (gap, label image)."""
     dev = require_cuda()
-    UV = torch.from_numpy(np.ascontiguousarray(uv, np.float64)).to(dev)
-    F = torch.from_numpy(np.ascontiguousarray(faces, np.int32).reshape(-1, 3)).to(dev)
-    lab = torch.from_numpy(np.ascontiguousarray(islands, np.int32)).to(dev)
+    UV = upload(uv, np.float64, dev)
+    F = upload(faces, np.int32, dev).reshape(-1, 3)
+    lab = upload(islands, np.int32, dev)
     g = min_gutter_device(UV, F, lab, int(lab.max().item()) + 1 if len(lab) else 0, int(res))
     img, _ = _gutter_raw(UV, F, lab, int(res), 1)
     return g, to_host(img)

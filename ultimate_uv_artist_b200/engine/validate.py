@@ -16,13 +16,14 @@ FMA contraction, so the verdicts match the reference bit for bit:
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 
 import numpy as np
 import torch
 
 from .. import _lib, meshops
-from ..device import require_cuda
+from ..device import require_cuda, upload
 
 ULP = 2.0 ** -24
 ULP_STRICT = 0.0
@@ -58,17 +59,19 @@ class DeviceValidation:
         self.dev = require_cuda(device)
         d = self.dev
         self.n, self.m = int(V.shape[0]), int(F.shape[0])
-        self.V = V if torch.is_tensor(V) else torch.from_numpy(np.ascontiguousarray(V, np.float64)).to(d)
-        self.UV = UV32 if torch.is_tensor(UV32) else torch.from_numpy(np.ascontiguousarray(UV32, np.float32)).to(d)
-        self.F = F if torch.is_tensor(F) else torch.from_numpy(np.ascontiguousarray(F, np.int32)).to(d)
         m4 = (max(self.m, 1) + 3) // 4 * 4
-        self.tflags = torch.zeros(m4, dtype=torch.uint8, device=d)
-        self.labels = torch.zeros(max(self.m, 1), dtype=torch.int32, device=d)
-        self.sa = torch.zeros(max(self.m, 1), dtype=torch.float64, device=d)
-        self.counts = torch.zeros(VC_N, dtype=torch.int64, device=d)
-        nb = C.c_int64()
-        _lib.check(L.uva_validate_scratch_bytes(self.n, self.m, int(grid), C.byref(nb)), "uva_validate_scratch_bytes")
-        self.scratch = torch.empty(max(int(nb.value), 256), dtype=torch.uint8, device=d)
+        # uploads and fills run on the stream of the pass
+        with (torch.cuda.stream(stream) if stream is not None else contextlib.nullcontext()):
+            self.V = V if torch.is_tensor(V) else upload(V, np.float64, d)
+            self.UV = UV32 if torch.is_tensor(UV32) else upload(UV32, np.float32, d)
+            self.F = F if torch.is_tensor(F) else upload(F, np.int32, d)
+            self.tflags = torch.zeros(m4, dtype=torch.uint8, device=d)
+            self.labels = torch.zeros(max(self.m, 1), dtype=torch.int32, device=d)
+            self.sa = torch.zeros(max(self.m, 1), dtype=torch.float64, device=d)
+            self.counts = torch.zeros(VC_N, dtype=torch.int64, device=d)
+            nb = C.c_int64()
+            _lib.check(L.uva_validate_scratch_bytes(self.n, self.m, int(grid), C.byref(nb)), "uva_validate_scratch_bytes")
+            self.scratch = torch.empty(max(int(nb.value), 256), dtype=torch.uint8, device=d)
         D = ValDesc()
         D.n, D.m, D.grid = self.n, self.m, int(grid)
         D.V, D.UV, D.F = self.V.data_ptr(), self.UV.data_ptr(), self.F.data_ptr()
@@ -122,12 +125,11 @@ def validate_uvs(v, f, uv, atlas=4096, padding=None, in_v=None, in_f=None, in_no
     each, every rank holding the whole mesh): each rank tests the overlap
     pairs of its band of the atlas, the overlap bits and pair counts are
     all-reduced, and every rank returns the same report."""
-    v = np.asarray(v, np.float64)
+    v = np.asarray(v)
     f = np.asarray(f, np.int64)
-    uv32 = np.asarray(uv, np.float32)
     from .. import shard as S
     rank, world = S.rank_world(group)
-    dv = DeviceValidation(v, f.astype(np.int32), uv32, shard=rank, nshards=world).run()
+    dv = DeviceValidation(v, f, np.asarray(uv), shard=rank, nshards=world).run()
     if world > 1:
         dv.merge(group)
     c = dv.host_counts()
@@ -152,7 +154,7 @@ def validate_uvs(v, f, uv, atlas=4096, padding=None, in_v=None, in_f=None, in_no
         if padding is not None:
             rep["gutter_ok"] = bool(rep["min_gutter_texels"] >= padding - 1e-6)
     if in_v is not None and in_f is not None:
-        in_v = np.asarray(in_v, np.float64)
+        in_v = np.asarray(in_v)
         in_f = np.asarray(in_f, np.int64)
         rep["triangle_count_preserved"] = bool(len(in_f) == len(f))
         if len(in_f) == len(f):
@@ -205,8 +207,8 @@ def _chart_overlap_flags(Un, T):
         L._uva_chart_sig = True
     dev = require_cuda()
     n, m = len(Un), len(T)
-    U = torch.from_numpy(Un).to(dev)
-    F = torch.from_numpy(T.astype(np.int32)).to(dev)
+    U = upload(Un, np.float64, dev)
+    F = upload(T, np.int32, dev)
     out = torch.zeros((m + 3) // 4 * 4, dtype=torch.uint8, device=dev)
     nb = C.c_int64()
     _lib.check(L.uva_validate_scratch_bytes(n, m, 0, C.byref(nb)), "uva_validate_scratch_bytes")

@@ -15,7 +15,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .device import require_cuda
+from .device import require_cuda, upload
 
 # element codes of uva_corners_equal
 _DTYPE_CODE = {np.dtype(np.float32): 0, np.dtype(np.float64): 1, np.dtype(np.float16): 2, np.dtype(np.uint8): 3,
@@ -148,10 +148,10 @@ def seam_report(V, F, UV, weld=None):
     nonmanifold_edge_groups, surface_area) of a mesh with per-vertex UVs."""
     L = _lib.lib()
     dev = require_cuda()
-    Vt = torch.from_numpy(np.ascontiguousarray(V, np.float64).reshape(-1, 3)).to(dev)
-    Ft = torch.from_numpy(np.ascontiguousarray(F, np.int64).reshape(-1, 3)).to(dev)
-    Ut = torch.from_numpy(np.ascontiguousarray(UV, np.float64).reshape(-1, 2)).to(dev)
-    Wt = None if weld is None else torch.from_numpy(np.ascontiguousarray(weld, np.int64).reshape(-1)).to(dev)
+    Vt = upload(V, np.float64, dev).reshape(-1, 3)
+    Ft = upload(F, np.int64, dev).reshape(-1, 3)
+    Ut = upload(UV, np.float64, dev).reshape(-1, 2)
+    Wt = None if weld is None else upload(weld, np.int64, dev).reshape(-1)
     n, m = int(Vt.shape[0]), int(Ft.shape[0])
     if Ut.shape[0] < n or (Wt is not None and Wt.shape[0] < n):
         raise IndexError("seam_report: uvs and weld keys need a row per vertex")
@@ -191,10 +191,10 @@ def corners_equal(a, fa, b, fb):
     dev = require_cuda()
     ar, w = _rows(a)
     br, _ = _rows(b)
-    ta = torch.from_numpy(ar).to(dev)
-    tb = torch.from_numpy(br).to(dev)
-    ia = torch.from_numpy(np.ascontiguousarray(fa, np.int64)).to(dev)
-    ib = torch.from_numpy(np.ascontiguousarray(fb, np.int64)).to(dev)
+    ta = upload(ar, ar.dtype, dev)
+    tb = upload(br, br.dtype, dev)
+    ia = upload(fa, np.int64, dev)
+    ib = upload(fb, np.int64, dev)
     res = torch.zeros(1, dtype=torch.int32, device=dev)
     _lib.check(L.uva_corners_equal(_p(ta), _DTYPE_CODE[a.dtype], len(ar), _p(ia), _p(tb), _DTYPE_CODE[b.dtype],
                                    len(br), _p(ib), int(fa.shape[0]), w, _p(res), _stream(dev)), "uva_corners_equal")
