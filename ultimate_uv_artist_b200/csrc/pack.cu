@@ -15,7 +15,9 @@
 // dilation is separable: rows, then columns.
 //
 // Runs (uva_pack_variants). A variant is a source turned by 0..3 quarter
-// turns (np.rot90). Its rows are stored as runs of set cells with the
+// turns (np.rot90). Its rows are stored as runs of set cells (a warp per row,
+// 32 cells per ballot: 33 us for the 72,000 rows of 180 charts x 4 turns, 217 us
+// byte by byte in one thread) with the
 // longest run of each row (pack.py:95-119), the set cells of the variant
 // (the "area" ordering key, pack.py:392) and the row with the longest run,
 // which the placement tests first.
@@ -23,24 +25,35 @@
 // Placement (uva_pack_place), one cooperative launch for all charts. The
 // page keeps, per cell, the free run to its right (R = 0: occupied) and, per
 // row, the longest free run. For every chart in turn (pack.py:312-359):
-//   A1. one thread per (row y, variant k) item tests every row of the
+//   A1. eight lanes per (row y, variant k) item test every row of the
 //       variant against the longest free run of the page row it would land
 //       on; the items that pass are bits in (y, k) order. Grid barrier.
 //   A2. blocks take the passing items by rank (block b: ranks b, b + nb, ...,
 //       so in increasing y). Per item every x is a bit of one thread: the
 //       widest run of the variant's longest-run row and of seven rows spread
 //       over its height must land on free runs at least as long (loads in
-//       flight together); the x left are candidates, tested whole in
-//       increasing x, one per warp, the lanes taking the rows. A fit lowers
-//       ybest[k] (atomic minimum); items below ybest[k] are skipped, and a
-//       block stops once every variant fits higher than its next item.
-//       ybest[k], bestx[k][ybest[k]] is the reference's first fit (smallest
-//       y, then smallest x, pack.py:124-156). Grid barrier.
+//       flight together); the x left are candidates, tested in increasing x:
+//       the first eight whole, one per warp, the lanes taking the rows; if
+//       none fits and more than eight are left, all of them on eight more
+//       rows, one candidate per thread; and so on. A fit lowers ybest[k]
+//       (atomic minimum). An item whose top edge y + h lies above that of a
+//       fit already found is left, also half-way, and a block stops once that
+//       holds for every variant: B would not choose it. For the variant that
+//       B chooses, (ybest, bestx) is the reference's first fit (smallest y,
+//       then smallest x, pack.py:124-156): no item of it is left. Grid barrier.
 //   B.  every block picks, from the same values, the variant of smallest
 //       (y + h) G + (x + w), the first on ties (pack.py:345-351); none: the
 //       attempt fails and every block returns.
 //   C.  blocks rebuild the free runs of the rows the chart covers; a grid
 //       barrier ends the chart.
+// The launch is bound by its slowest item, a chain of L2 round trips in one
+// block, not by bandwidth: 52 us per chart with eight whole checks a round to
+// the end of the candidates, one thread per item in A1 and 64-bit ranks found
+// by binary search; 28 with the rows in between (many x pass eight filter
+// rows and fail later: the slowest block's wait fell from 31 to 9 us a chart),
+// 21 with eight lanes per item and ballots for the ranks, 20 with the top edge
+// bound (180 charts, 2048 x 2048 page, 26 attempts: 244 -> 99 ms).
+//
 // Values written inside the launch are read with ld.global.cg (L2), so no
 // block sees a stale line of its own L1. The barrier spins a bounded time
 // (two seconds) and reports a timeout in the status instead of waiting for
@@ -230,32 +243,46 @@ __global__ void k_pk_runs(int64_t nrows, int32_t nvar, const int64_t* var_row, c
                           int32_t* run_ofs, int32_t* row_need, unsigned long long* var_area,
                           unsigned long long* var_key, int32_t* run_a, int32_t* run_b, int64_t run_cap,
                           int32_t* status) {
-    GRID_STRIDE(r, nrows) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nwarps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+    for (int64_t r = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); r < nrows; r += nwarps) {
         const int32_t v = find_seg(var_row, nvar, r);
         const Variant vr = variant_of(v, var_src, var_turn, hw);
         const int32_t i = static_cast<int32_t>(r - var_row[v]);
         const int32_t h0 = hw[2 * vr.src], w0 = hw[2 * vr.src + 1];
         const uint8_t* m = mask + mofs[vr.src];
-        int32_t cnt = 0, need = 0, cells = 0;
+        int32_t cnt = 0, need = 0, cells = 0, start = -1;   // start: of the open run
         int64_t q = FILL ? run_ofs[r] : 0;
-        int32_t j = 0;
-        while (j < vr.w) {
-            if (turned_cell(m, h0, w0, vr.turn, i, j)) {
-                const int32_t s = j;
-                while (j < vr.w && turned_cell(m, h0, w0, vr.turn, i, j)) ++j;
-                if (FILL) {
-                    if (q < run_cap) { run_a[q] = s; run_b[q] = j - 1; }
-                    else atomicOr(status, 1);
-                    ++q;
+        auto run = [&](int32_t a, int32_t b) {
+            if (FILL && lane == 0) {
+                if (q < run_cap) { run_a[q] = a; run_b[q] = b; }
+                else atomicOr(status, 1);
+            }
+            ++q;
+            ++cnt;
+            cells += b - a + 1;
+            need = max(need, b - a + 1);
+        };
+        for (int32_t j0 = 0; j0 < vr.w; j0 += 32) {
+            const int32_t j = j0 + lane;
+            const unsigned set = __ballot_sync(0xffffffffu, j < vr.w && turned_cell(m, h0, w0, vr.turn, i, j));
+            // the word's edges one after the other: the next set bit opens a
+            // run, the next clear bit ends it
+            for (unsigned rest = 0xffffffffu; rest;) {
+                const unsigned t = (start < 0 ? set : ~set) & rest;
+                if (!t) break;
+                const int32_t b = __ffs(t) - 1;
+                if (start < 0) {
+                    start = j0 + b;
+                } else {
+                    run(start, j0 + b - 1);
+                    start = -1;
                 }
-                ++cnt;
-                cells += j - s;
-                need = max(need, j - s);
-            } else {
-                ++j;
+                rest = 0xfffffffeu << b;
             }
         }
-        if (!FILL) {
+        if (start >= 0) run(start, vr.w - 1);
+        if (!FILL && lane == 0) {
             run_ofs[r] = cnt;
             row_need[r] = need;
             if (cells) atomicAdd(var_area + v, static_cast<unsigned long long>(cells));
@@ -357,16 +384,61 @@ struct ChartVariants {
 __device__ __forceinline__ bool warp_fits(const int32_t* R, const int32_t* run_ofs, const int32_t* run_a,
                                           const int32_t* run_b, int32_t G, int32_t y, int32_t x, int32_t h,
                                           int64_t r0, int lane) {
+    for (int32_t j0 = 0; j0 < h; j0 += 32) {   // 32 rows at a time: most of those that fail do so early
+        const int32_t j = j0 + lane;
+        bool ok = true;
+        if (j < h) {
+            const int32_t* Rrow = R + static_cast<int64_t>(y + j) * G + x;
+            const int32_t q1 = __ldg(run_ofs + r0 + j + 1);
+            for (int32_t q = __ldg(run_ofs + r0 + j); q < q1; ++q) {
+                const int32_t qa = __ldg(run_a + q);
+                ok &= __ldcg(Rrow + qa) >= __ldg(run_b + q) - qa + 1;
+            }
+        }
+        if (!__all_sync(0xffffffffu, ok)) return false;
+    }
+    return true;
+}
+
+// Position of the n-th (from 0) set bit of a word, the same on every lane.
+__device__ __forceinline__ int nth_bit(unsigned word, int32_t n, int lane) {
+    return __ffs(__ballot_sync(0xffffffffu, (word >> lane & 1u) && __popc(word & ((1u << lane) - 1u)) == n)) - 1;
+}
+
+// Do the rows b, b + step, b + 2 step, ... (kSpread of them) of the variant
+// fit with its corner at (x, y)? For one thread, whose neighbours ask for the
+// neighbouring x: every load is one or two lines for the warp.
+constexpr int kSpread = 8;
+__device__ __forceinline__ bool rows_fit(const int32_t* R, const int32_t* run_ofs, const int32_t* run_a,
+                                         const int32_t* run_b, int32_t G, int32_t y, int32_t x, int32_t h,
+                                         int64_t r0, int32_t b, int32_t step) {
+    int32_t q0[kSpread], q1[kSpread], qa[kSpread], len[kSpread], fr[kSpread];
+#pragma unroll
+    for (int i = 0; i < kSpread; ++i) {
+        const int32_t j = min(b + i * step, h - 1);
+        q0[i] = __ldg(run_ofs + r0 + j);
+        q1[i] = __ldg(run_ofs + r0 + j + 1);
+    }
+#pragma unroll
+    for (int i = 0; i < kSpread; ++i) {
+        qa[i] = q0[i] < q1[i] ? __ldg(run_a + q0[i]) : 0;
+        len[i] = q0[i] < q1[i] ? __ldg(run_b + q0[i]) - qa[i] + 1 : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < kSpread; ++i)
+        fr[i] = __ldcg(R + static_cast<int64_t>(y + min(b + i * step, h - 1)) * G + x + qa[i]);
     bool ok = true;
-    for (int32_t j = lane; j < h; j += 32) {
-        const int32_t* Rrow = R + static_cast<int64_t>(y + j) * G + x;
-        const int32_t q1 = __ldg(run_ofs + r0 + j + 1);
-        for (int32_t q = __ldg(run_ofs + r0 + j); q < q1; ++q) {
-            const int32_t qa = __ldg(run_a + q);
-            ok &= __ldcg(Rrow + qa) >= __ldg(run_b + q) - qa + 1;
+#pragma unroll
+    for (int i = 0; i < kSpread; ++i) ok &= fr[i] >= len[i];
+#pragma unroll
+    for (int i = 0; i < kSpread; ++i) {   // rows of more than one run
+        const int32_t* Rrow = R + static_cast<int64_t>(y + min(b + i * step, h - 1)) * G + x;
+        for (int32_t q = q0[i] + 1; ok && q < q1[i]; ++q) {
+            const int32_t a = __ldg(run_a + q);
+            ok = __ldcg(Rrow + a) >= __ldg(run_b + q) - a + 1;
         }
     }
-    return __all_sync(0xffffffffu, ok);
+    return ok;
 }
 
 // Dynamic shared memory: G free-run ints, then G occupancy bytes.
@@ -432,32 +504,34 @@ __global__ void __launch_bounds__(kTB, 4) k_pk_place(PlaceMulti pm) {
         }
         __syncthreads();
         // ---- A1: the items (y, k) whose rows all fit the longest free runs of
-        // the page rows below them, one thread per item, as bits in y-major order
+        // the page rows below them, as bits in y-major order
         const int64_t items = static_cast<int64_t>(nk) * G;
         unsigned* cb = a.cand + (p & 1) * a.cand_words;
         for (int32_t i = threadIdx.x; i < G; i += blockDim.x) s_R[i] = __ldcg(a.rowmax + i);   // s_R: rowmax here
         __syncthreads();
-        // a warp owns the word of its 32 items (it = warp-aligned base + lane)
-        for (int64_t base = (bid * static_cast<int64_t>(blockDim.x) + threadIdx.x) & ~int64_t(31);
-             base < items; base += static_cast<int64_t>(nb) * blockDim.x) {
-            const int64_t it = base + lane;
+        // eight lanes per item, four items per warp: a lane takes four rows of 32
+        for (int64_t base = 4 * ((bid * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5); base < items;
+             base += static_cast<int64_t>(nb) * (kTB / 8)) {
+            const int32_t it = static_cast<int32_t>(base) + (lane >> 3);
             bool ok = false;
             if (it < items) {
-                const int32_t y = static_cast<int32_t>(it / nk), k = static_cast<int32_t>(it - static_cast<int64_t>(y) * nk);
-                const int32_t h = cv.h[k];
+                const int32_t y = it / nk, k = it - y * nk, h = cv.h[k];
                 if (h > 0 && y <= G - h) {
                     const int32_t* need = a.row_need + cv.r0[k];
                     const int32_t* rm = s_R + y;
                     ok = true;
-                    for (int32_t j = 0; j < h && ok; j += 4) {   // four rows a step, the last row again past the end
+                    for (int32_t j = 4 * (lane & 7); j < h && ok; j += 32) {   // the last row again past the end
                         const int32_t j1 = min(j + 1, h - 1), j2 = min(j + 2, h - 1), j3 = min(j + 3, h - 1);
                         ok = (__ldg(need + j) <= rm[j]) & (__ldg(need + j1) <= rm[j1]) & (__ldg(need + j2) <= rm[j2]) &
                              (__ldg(need + j3) <= rm[j3]);
                     }
                 }
             }
-            const unsigned bits = __ballot_sync(0xffffffffu, ok);
-            if (lane == 0 && bits) cb[base >> 5] = bits;
+            const unsigned no = ~__ballot_sync(0xffffffffu, ok);
+            unsigned bits = 0;   // four items; base is a multiple of 4: one word
+#pragma unroll
+            for (int i = 0; i < 4; ++i) bits |= static_cast<unsigned>((no >> (8 * i) & 255u) == 0) << i;
+            if (lane == 0 && bits) atomicOr(cb + (base >> 5), bits << (base & 31));
         }
         if (!grid_sync(a.bar, nb)) {
             if (bid == 0 && threadIdx.x == 0) atomicOr(a.status, 2);
@@ -465,7 +539,7 @@ __global__ void __launch_bounds__(kTB, 4) k_pk_place(PlaceMulti pm) {
         }
         // ---- A2: first fit of every variant over the items of A1, in
         // increasing (y, k); block b takes the items of rank b, b + nb, ...
-        int64_t carry = 0;
+        int32_t carry = 0;   // items before this tile (nk G < 2^31)
         bool all_done = false;
         int r_par = 0;
         for (int64_t w0 = 0; w0 < a.cand_words && !all_done; w0 += blockDim.x) {
@@ -488,17 +562,15 @@ __global__ void __launch_bounds__(kTB, 4) k_pk_place(PlaceMulti pm) {
             s_word[threadIdx.x] = word;
             s_pref[threadIdx.x] = wbase + incl - __popc(word);   // exclusive
             __syncthreads();
-            const int64_t r_first = carry + ((static_cast<int64_t>(bid) - carry) % nb + nb) % nb;
-            for (int64_t r = r_first; r < carry + total; r += nb) {
-                const int32_t rr = static_cast<int32_t>(r - carry);
-                int32_t lo = 0, hi = kTB - 1;   // the last thread whose exclusive prefix is <= rr
-                while (lo < hi) {
-                    const int32_t mid = (lo + hi + 1) >> 1;
-                    if (s_pref[mid] <= rr) lo = mid; else hi = mid - 1;
-                }
-                const int bit = __fns(s_word[lo], 0, rr - s_pref[lo] + 1);
-                const int64_t it = (w0 + lo) * 32 + bit;
-                const int32_t y = static_cast<int32_t>(it / nk), k = static_cast<int32_t>(it - static_cast<int64_t>(y) * nk);
+            const int32_t nbl = static_cast<int32_t>(nb), back = carry % nbl;
+            for (int32_t rr = static_cast<int32_t>(bid) - back + (static_cast<int32_t>(bid) < back ? nbl : 0); rr < total; rr += nbl) {
+                // the last thread whose exclusive prefix is <= rr, in two ballots
+                constexpr int kPer = kTB / 32;
+                const int32_t top = __popc(__ballot_sync(0xffffffffu, s_pref[kPer * lane] <= rr)) - 1;
+                const int32_t in = __popc(__ballot_sync(0xffffffffu, lane < kPer && s_pref[kPer * top + min(lane, kPer - 1)] <= rr)) - 1;
+                const int32_t lo = kPer * top + in;
+                const int32_t it = static_cast<int32_t>(w0 + lo) * 32 + nth_bit(s_word[lo], rr - s_pref[lo], lane);
+                const int32_t y = it / nk, k = it - y * nk;
                 const int32_t h = cv.h[k], w = cv.w[k];
                 const int64_t r0 = cv.r0[k];
                 if (threadIdx.x == 0) { s_best = kNone; s_slots = 0; }
@@ -517,16 +589,22 @@ __global__ void __launch_bounds__(kTB, 4) k_pk_place(PlaceMulti pm) {
                         cand |= static_cast<unsigned>(ok) << m;
                     }
                 }
-                // skip: a higher row already fits this variant; done: a higher
-                // row fits every variant (this block's later items are lower)
+                // top: the lowest top edge of a fit found so far, by any block.
+                // The choice takes the lowest top edge, so an item whose own
+                // lies above that has no say (and none of this block's later
+                // ones, once that holds for every variant).
                 int32_t* syb = s_yb[r_par];
                 r_par ^= 1;
                 if (threadIdx.x < nk) syb[threadIdx.x] = __ldcg(yb + threadIdx.x);
                 __syncthreads();
-                bool done = true;
-                for (int32_t kk = 0; kk < nk; ++kk) done &= cv.h[kk] == 0 || syb[kk] < y;
-                if (done) { all_done = true; break; }
-                if (syb[k] < y) continue;
+                int32_t top_edge = kNone, hmin = kNone;
+                for (int32_t kk = 0; kk < nk; ++kk) {
+                    if (cv.h[kk] == 0) continue;
+                    hmin = min(hmin, cv.h[kk]);
+                    if (syb[kk] != kNone) top_edge = min(top_edge, syb[kk] + cv.h[kk]);
+                }
+                if (y + hmin > top_edge) { all_done = true; break; }
+                if (y + h > top_edge) continue;
                 // the other filters, all loads of one slot in flight together
                 for (unsigned live = cand; live; live &= live - 1) {
                     const int32_t m = __ffs(live) - 1;
@@ -537,45 +615,55 @@ __global__ void __launch_bounds__(kTB, 4) k_pk_place(PlaceMulti pm) {
                         ok &= __ldcg(a.R + static_cast<int64_t>(y + cv.fy[k][f]) * G + cv.fa[k][f] + x) >= cv.fl[k][f];
                     if (!ok) cand &= ~(1u << m);
                 }
-                // slot by slot in increasing x, the candidates, one per warp,
-                // checked whole by the warp's lanes; the first slot with a fit ends it
+                // slot by slot in increasing x: the first kWarps candidates, one
+                // per warp, are checked whole by the warp's lanes; when none
+                // fits and more are left than another such round takes, every
+                // candidate is tested on kSpread more rows spread over the
+                // height. The first slot with a fit ends it, or another block's fit with
+                // a lower top edge.
                 if (cand) atomicOr(&s_slots, cand);
                 __syncthreads();
                 unsigned slots = s_slots;
+                const int32_t step = (h + kSpread - 1) / kSpread;
                 bool found = false;
-                while (slots) {
+                while (slots && !found) {
                     const int32_t m = __ffs(slots) - 1;
                     slots &= slots - 1;
-                    // word `warp` holds the candidates m * blockDim.x + warp * 32 + lane
-                    const unsigned bits = __ballot_sync(0xffffffffu, (cand >> m) & 1u);
-                    if (lane == 0) s_cand[warp] = bits;
-                    __syncthreads();
-                    const unsigned word = lane < kWarps ? s_cand[lane] : 0u;
-                    int32_t incl = __popc(word);
+                    const int32_t xt = m * static_cast<int32_t>(blockDim.x) + static_cast<int32_t>(threadIdx.x);
+                    bool live = (cand >> m) & 1u;
+                    for (int32_t b = 0;; ++b) {
+                        // word `warp` holds the candidates m * blockDim.x + warp * 32 + lane
+                        const unsigned bits = __ballot_sync(0xffffffffu, live);
+                        const int32_t yo = threadIdx.x < nk ? __ldcg(yb + threadIdx.x) : kNone;   // other blocks' fits
+                        if (lane == 0) s_cand[warp] = bits;
+                        __syncthreads();
+                        const unsigned word = lane < kWarps ? s_cand[lane] : 0u;
+                        int32_t incl = __popc(word);
 #pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-                        if (lane >= o) incl += t;
-                    }
-                    const int32_t ncand = __shfl_sync(0xffffffffu, incl, 31);
-                    for (int32_t base = 0; base < ncand; base += kWarps) {
-                        const int32_t r = base + warp;
+                        for (int o = 1; o < kWarps; o <<= 1) {
+                            const int32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+                            if (lane >= o) incl += t;
+                        }
+                        const int32_t ncand = __shfl_sync(0xffffffffu, incl, kWarps - 1);
                         bool ok = false;
-                        if (r < ncand) {
-                            const unsigned above = __ballot_sync(0xffffffffu, incl > r);
+                        if (warp < ncand) {
+                            const unsigned above = __ballot_sync(0xffffffffu, lane < kWarps && incl > warp);
                             const int wi = __ffs(above) - 1;
                             const unsigned wbits = __shfl_sync(0xffffffffu, word, wi);
                             const int32_t before = __shfl_sync(0xffffffffu, incl - __popc(word), wi);
-                            const int bit = __fns(wbits, 0, r - before + 1);
+                            const int bit = nth_bit(wbits, warp - before, lane);
                             const int32_t x = m * static_cast<int32_t>(blockDim.x) + wi * 32 + bit;
                             ok = warp_fits(a.R, a.run_ofs, a.run_a, a.run_b, G, y, x, h, r0, lane);
                             if (ok && lane == 0) atomicMin(&s_best, x);
                         }
-                        found = __syncthreads_or(ok && lane == 0);
-                        if (found) break;
+                        // this thread's candidate is one of those
+                        const int32_t base = __shfl_sync(0xffffffffu, incl - __popc(word), warp);
+                        if (base + __popc(bits & ((1u << lane) - 1u)) < kWarps) live = false;
+                        found = __syncthreads_or((ok && lane == 0) || (yo != kNone && yo + cv.h[threadIdx.x] < y + h));
+                        if (found || ncand <= kWarps) break;
+                        if (ncand > 2 * kWarps && b < step && live)
+                            live = rows_fit(a.R, a.run_ofs, a.run_a, a.run_b, G, y, xt, h, r0, b, step);
                     }
-                    if (found) break;
-                    __syncthreads();   // s_cand is rewritten for the next slot
                 }
                 if (threadIdx.x == 0 && s_best != kNone) {
                     a.bestx[static_cast<int64_t>(k) * G + y] = s_best;
@@ -827,12 +915,12 @@ extern "C" int uva_pack_masks(const uva_pack_attempt* a, void* stream) {
                                                               a->mask);
     }
     if (a->nrows > 0) {
-        k_pk_runs<false><<<blocks_for(a->nrows), kTB, 0, st>>>(
+        k_pk_runs<false><<<blocks_for(32 * a->nrows), kTB, 0, st>>>(
             a->nrows, nvar, a->var_row, a->var_src, a->var_turn, a->hw, a->mofs, a->mask, a->run_ofs, a->row_need,
             reinterpret_cast<unsigned long long*>(a->var_area), reinterpret_cast<unsigned long long*>(a->var_key),
             nullptr, nullptr, 0, a->status + 2);
         xscan<int32_t>(a->run_ofs, a->run_ofs, s.sums, nullptr, a->nrows + 1, st);
-        k_pk_runs<true><<<blocks_for(a->nrows), kTB, 0, st>>>(
+        k_pk_runs<true><<<blocks_for(32 * a->nrows), kTB, 0, st>>>(
             a->nrows, nvar, a->var_row, a->var_src, a->var_turn, a->hw, a->mofs, a->mask, a->run_ofs, a->row_need,
             nullptr, nullptr, a->run_a, a->run_b, a->run_cap, a->status + 2);
     }
