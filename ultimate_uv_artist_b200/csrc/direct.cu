@@ -5,7 +5,7 @@
 // Why: a chart is a planar graph, so in breadth-first order its matrix has a
 // narrow skyline (about the square root of n). An 8,061-vertex disk has
 // 3,779 blocks of 16 x 16 in its factor: 27 million multiply-adds and 7.7 MB,
-// where the FP32 two-level CG needed 1,416 iterations of LSCM (and some 40
+// where the FP32 two-level CG needs 1,416 iterations of LSCM (and some 40
 // per ARAP step) whose cost is barriers and L2 round trips. The factor is
 // exact to FP64 round-off, so one solve per global step meets the tolerance
 // that the FP64 residual check asks for; ARAP factors once per call and
@@ -17,14 +17,27 @@
 //             block column of every block row, number of blocks.
 //   k_direct  block LDL^H, left-looking by block columns of 16: S_IK = A_IK -
 //             sum_M G_IM L_KM^H (G = L D kept in a ring of 16 x 16 blocks),
-//             D_K inverted by one warp, L_IK = S_IK D_K^-1. The products run
-//             on the FP64 tensor instruction (m8n8k4). LSCM factors the
+//             D_K inverted by the CTA, an element per thread, 2 x 2 pivots),
+//             L_IK = S_IK D_K^-1. The products run on the FP64 tensor
+//             instruction (m8n8k4). LSCM factors the
 //             complex Hermitian n x n form of its (u, v) system, ARAP the
 //             real one.
 //   solves    forward and backward substitution with one barrier per block:
 //             a group of 16 threads owns every sixteenth block row and keeps
 //             its right-hand side in registers; the factor streams through a
 //             ring of shared-memory stages (cp.async.bulk, mbarriers).
+//
+// What bounds it: the largest island, one CTA from end to end of the launch.
+// Its factor is a chain of block columns with some 16 dependent L2 round trips
+// (about 800 cycles each) a column: 8.1 ms of the 11.5 ms LSCM launch of 2,000
+// islands (8,061 vertices the largest). Its substitutions are a chain of 504
+// steps of 960 cycles, three fifths of them shared-memory loads and the FP64
+// sums, the rest the hand-over of the block and its barrier: 11.7 ms of the
+// 29.9 ms ARAP launch of 20 iterations; local step, right-hand side, residual
+// and line search take 11.4, the factor 4.5. With CG: 40.0 ms LSCM, 39.6 ARAP.
+// Tried and slower: fragments of L prefetched in registers from global memory
+// (45 ms ARAP), block x vector on the tensor instruction (36), the same layout
+// with scalar sums and two feeding warps (29.9 ARAP, but 12.7 LSCM).
 //
 // Blocks are stored column by column with an XOR swizzle (element (r, c) at
 // 16 c + (r ^ c)): a forward step reads a column over 16 lanes, a backward
@@ -879,7 +892,7 @@ __global__ void __launch_bounds__(kNT, 2) k_direct(uva_batch b, uva_solve_params
         const int64_t need = (static_cast<int64_t>(total) + 256) * BB * 8 + static_cast<int64_t>(npad) * 16 * (CP ? 1 : 3);
         bool done = false;
         const long long t0 = global_ns();
-        if (info[0] && need <= room) {
+        if ((info[0] & 1) && need <= room) {
             const int32_t* first = band_first(b, I.v0, I.id);
             I.pin = b.vert_row[I.v0 + b.pins[3 * I.id]];
             const int q0 = b.pins[3 * I.id + 1], q1 = b.pins[3 * I.id + 2];

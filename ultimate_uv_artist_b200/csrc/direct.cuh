@@ -10,8 +10,9 @@ constexpr int kDirectMaxN = 16384;   // vertices of an island (band positions fi
 constexpr int kWorkNext = 4, kWorkLeft = 5;
 
 // uva_batch.band: position of every solver row (n), first block column of
-// every block row (n / 16 + nc), then 4 ints per island: factor is possible,
-// blocks, widest row, solved by the last launch.
+// every block row (n / 16 + nc), then 4 ints per island: a factor is possible
+// (bit 0) and the coarse operators of CG are built (bit 1), blocks, widest
+// row, solved by the last launch.
 __host__ __device__ __forceinline__ int32_t* band_first(const uva_batch& b, int v0, int isl) {
     return b.band + b.n + v0 / 16 + isl;
 }

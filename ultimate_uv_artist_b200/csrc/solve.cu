@@ -12,6 +12,11 @@
 //    x_j) + [i == pin] wpin x_i, from FP32 edge weights in a sliced-ELL layout.
 //    Zero row sums then hold exactly in any precision, which keeps the
 //    near-singular soft-pinned system well posed in FP32.
+//  * Islands of up to 16,384 vertices are solved by FP64 factors (direct.cu,
+//    launched first); what follows holds for the others: larger or wide ones,
+//    those whose factor does not fit its scratch or has a zero pivot, ARAP
+//    calls of fewer than kDirectMinIters iterations, and callers without the
+//    factor's scratch.
 //  * Mixed precision: each global step solves L x = b with FP32 Jacobi-PCG
 //    corrections and recomputes the residual b - L x in FP64 (iterative
 //    refinement) until ||b - L x|| <= tol ||b|| per column, checked in FP64.
@@ -1765,16 +1770,25 @@ static_assert(sizeof(double) * kCoarseSmemN * kCoarseSmemN <= kCoarseSmem, "real
 constexpr int kCoarseSmallM = 32;
 constexpr size_t kCoarseSmallSmem = sizeof(double2) * kCoarseSmallM * kCoarseSmallM;   // 16 KB
 
+// Only the CG path reads the operators, so with an elimination order (b.band)
+// the set-up leaves out the islands that a factor can solve, and a solve
+// launches this again with `left` set, for the islands it is about to give to
+// CG without one (ARAP calls of few iterations, no scratch, a zero pivot):
+// 1.8 ms of the set-up of 2,000 islands, 0.31 of one of 6,100 triangles;
+// the launch that finds nothing to do takes 2 us (one island) to 7.
 template <int NT>
-__global__ void __launch_bounds__(NT) k_coarse(uva_batch b, int first, int count) {
+__global__ void __launch_bounds__(NT) k_coarse(uva_batch b, int first, int count, int left) {
     extern __shared__ __align__(16) double wsm[];
     __shared__ double2 colk2[256], rowk2[256];   // pivot column / row (complex; the real pass uses 256 doubles of each)
     double* colk = reinterpret_cast<double*>(colk2);
     double* rowk = reinterpret_cast<double*>(rowk2);
     if (static_cast<int>(blockIdx.x) >= count) return;
+    if (left && b.direct && b.work[kWorkLeft] == 0) return;
     const int isl = b.order[first + blockIdx.x];   // largest islands first (b.order is by size)
     const int agg = b.agg_rows[isl];
     if (agg <= 0) return;
+    int32_t* info = b.band ? band_info(b, isl) : nullptr;
+    if (info && (left ? (info[0] & 2) || (b.direct && info[3]) : info[0] & 1)) return;
     const int v0 = b.vofs[isl], n = b.vofs[isl + 1] - v0, s0 = b.sofs[isl];
     const int M = (n + agg - 1) / agg;
     const int co = b.cofs[isl];
@@ -1818,6 +1832,7 @@ __global__ void __launch_bounds__(NT) k_coarse(uva_batch b, int first, int count
     gauss_jordan(W, M, colk, rowk);
     store_half_scaled(W, M, coarse_stride(M, 2), b.coarse_a + co, colk);
     __syncthreads();
+    if (info && threadIdx.x == 0) info[0] |= 2;   // read by every thread before the barriers above
     // ---- LSCM (free unknowns only; the pins are fixed)
     const int pv0 = b.pins[3 * isl + 1], pv1 = b.pins[3 * isl + 2];
     if (pv0 < 0 || pv1 < 0) return;
@@ -1863,6 +1878,20 @@ __global__ void __launch_bounds__(NT) k_coarse(uva_batch b, int first, int count
     }
     gauss_jordan_c(Wc, M, colk2, rowk2);
     store_complex_scaled(Wc, M, coarse_stride(M, 2), b.coarse_l + 4 * static_cast<size_t>(co), colk);
+}
+
+cudaError_t ensure_coarse_attr();
+
+// Whole-CTA classes (W, G, A: islands above 2048 vertices), then the smaller
+// ones (aggregates of 64 rows: at most 32 x 32 operators).
+cudaError_t launch_coarse(const uva_batch* b, bool left, cudaStream_t s) {
+    if (!b->coarse_a || !b->coarse_l || !b->coarse_work) return cudaSuccess;
+    const cudaError_t e = ensure_coarse_attr();   // 222 KB of dynamic shared memory
+    if (e != cudaSuccess) return e;
+    const int big = std::min(std::max(b->class_ofs[2], 0), b->nc), rest = b->nc - big;
+    if (big > 0) k_coarse<1024><<<big, 1024, kCoarseSmem, s>>>(*b, 0, big, left);
+    if (rest > 0) k_coarse<256><<<rest, 256, kCoarseSmallSmem, s>>>(*b, big, rest, left);
+    return cudaGetLastError();
 }
 
 cudaError_t ensure_coarse_attr() {
@@ -1950,6 +1979,10 @@ int launch_islands(const uva_batch* b, const uva_solve_params* prm, cudaStream_t
     if (b->direct) {   // the islands it leaves (info[3] == 0) are solved below
         const int rc = uva_direct_launch(b, prm, OP == OP_LSCM, s);
         if (rc != UVA_OK) return rc;
+    }
+    if (b->band) {   // coarse operators that the set-up left out and these islands need
+        e = launch_coarse(b, true, s);
+        if (e != cudaSuccess) return uva_cuda_status(e, "uva_islands/coarse");
     }
     const int big = b->class_ofs[2];                        // islands that take a whole CTA
     const int small = b->class_ofs[4] - b->class_ofs[2];    // islands for sub-teams / warps
@@ -2287,16 +2320,8 @@ extern "C" int uva_batch_setup(uva_batch* b, void* stream) {
         const int rc = uva_direct_order(b, s);
         if (rc != UVA_OK) return rc;
     }
-    if (b->coarse_a && b->coarse_l && b->coarse_work) {
-        const cudaError_t e = ensure_coarse_attr();   // 128 KB of dynamic shared memory
-        if (e != cudaSuccess) return uva_cuda_status(e, "uva_batch_setup/coarse attribute");
-        // whole-CTA classes (W, G, A: islands above 2048 vertices), then the
-        // smaller ones (aggregates of 64 rows: at most 32 x 32 operators)
-        const int big = std::min(std::max(b->class_ofs[2], 0), b->nc), rest = b->nc - big;
-        if (big > 0) k_coarse<1024><<<big, 1024, kCoarseSmem, s>>>(*b, 0, big);
-        if (rest > 0) k_coarse<256><<<rest, 256, kCoarseSmallSmem, s>>>(*b, big, rest);
-        UVA_CHECK_LAUNCH("uva_batch_setup/coarse");
-    }
+    const cudaError_t e = launch_coarse(b, false, s);
+    if (e != cudaSuccess) return uva_cuda_status(e, "uva_batch_setup/coarse");
     return UVA_OK;
 }
 

@@ -6,10 +6,12 @@ and keeps every per-island array in HBM: frames, weights, the sliced-ELL
 Laplacian, UVs and solver scratch. All solver calls run on one CUDA stream and
 never synchronise the host.
 
-Memory: about 80 bytes per triangle plus about 180 bytes per vertex
-(UVs, solver vectors, sliced-ELL slots) and 20 bytes per squared coarse
-aggregate, so a 180 GB B200 holds batches of several hundred million
-triangles.
+Memory: about 80 bytes per triangle plus about 184 bytes per vertex
+(UVs, solver vectors, sliced-ELL slots, elimination order) and 20 bytes per
+squared coarse aggregate, so a 180 GB B200 holds batches of several hundred
+million triangles. A solve also takes the direct solver's scratch from torch's
+allocator while it runs: one part per resident CTA (two per SM), sized for the
+largest islands up to 16,384 vertices (at most 31 MB each for ARAP, 60 for LSCM).
 """
 from __future__ import annotations
 
@@ -26,7 +28,9 @@ from ._lib import check, ptr
 # ARAP solves each global step to 2e-7 relative residual per column: at 1e-6
 # the UVs after 20 outer iterations drift up to 3e-5 (relative to the chart's
 # UV extent) from exact solves on 2,000 uneven islands; at 2e-7 they stay
-# below 4e-6, for about 13 % more CG iterations. Inner FP32 solves aim at a
+# below 4e-6, for about 13 % more CG iterations (islands of up to 16,384
+# vertices are solved by FP64 factors, to some 1e-13, and only checked against
+# it; figures here are those of the CG path). Inner FP32 solves aim at a
 # 1e-5 reduction (or the final tolerance): fewer FP64 restarts than 1e-3.
 # LSCM solves to 1e-8: on the same islands (12 size-stratified ones against
 # the FP64 oracle) the LSCM UVs stay within 4.5e-7 of exact solves and the

@@ -4,8 +4,9 @@ LSCM initialisation and ARAP local/global refinement).
 Same functions and signatures (engine/param.py:15-551). The numerical work
 runs in the uva_b200 CUDA kernels:
 
-* ``lscm``: conformal energy with the far-pair hard pins, solved by FP32 PCG
-  with FP64 residual refinement to 1e-9 relative residual;
+* ``lscm``: conformal energy with the far-pair hard pins, solved by an FP64
+  factor (up to 16,384 vertices) or by FP32 PCG with FP64 residual refinement,
+  to 1e-9 relative residual;
 * ``refine(method="arap")``: the persistent island kernel with param
   semantics (per-chart pin weight, flip-safe step only from a flip-free
   start, relative-energy stop); each global step is solved to 1e-10 relative
