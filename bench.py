@@ -37,7 +37,6 @@ METRIC = "ARAP tris/sec @1e-6 resid, batched-FP32+FP64-refine"
 UNIT = "tri-iters/s"
 ITERS = 20
 ISLANDS = 2000
-TRAFFIC_ARAP = 32.78e9   # bytes per ARAP launch of the default workload (ncu dram__bytes_read + write)
 
 
 def _args():
@@ -157,34 +156,48 @@ def _island_stats(batch):
     return n, t, n + off
 
 
-def arap_bytes(n, t, nnz, st):
+def factor_blocks(db):
+    """16 x 16 blocks in the FP64 factor of every island that the last solve
+    took directly, 0 for the islands solved by CG."""
+    nc, n = db.nc, db.n
+    at = n + n // 16 + nc
+    info = db.band[at:at + 4 * nc].cpu().numpy().reshape(nc, 4).astype(np.int64)
+    return np.where(info[:, 3] != 0, info[:, 1], 0)
+
+
+def arap_bytes(n, t, nnz, st, blocks):
     """Algorithmic bytes of one ARAP launch (fp32 data, int32 indices):
     per outer iteration 48 t + 40 n (local step, RHS, line search), per CG
     iteration 8 nnz + 56 n, per FP64 residual 8 nnz + 52 n; K and R as
-    executed. Also the compulsory bytes (K = R = 1 per outer iteration)."""
+    executed. An island solved by its FP64 factor (K = 0) writes and reads the
+    factor once to build it and reads it twice per solve (R solves). Also the
+    compulsory bytes (K = R = 1 per outer iteration)."""
     it = st["outer_iters"].astype(np.float64)
     K = st["cg_iters"].astype(np.float64)
     R = st["refinements"].astype(np.float64)
     per_outer = 48.0 * t + 40.0 * n
     cg = 8.0 * nnz + 56.0 * n
     rf = 8.0 * nnz + 52.0 * n
-    full = float((it * per_outer + K * cg + R * rf).sum())
+    factor = 2048.0 * blocks
+    full = float((it * per_outer + K * cg + R * rf + factor * (2.0 + 2.0 * R)).sum())
     comp = float((it * (per_outer + cg + rf)).sum())
     return full, comp
 
 
-def lscm_bytes(n, nnz, nbnd, st):
+def lscm_bytes(n, nnz, nbnd, st, blocks):
     """Algorithmic bytes of one LSCM launch: the PCG formula on the 2n
     unknowns (u, v) of each island, whose matrix holds the Laplacian twice
     plus the boundary coupling (nnz_H = 2 nnz + 4 boundary vertices): per CG
     iteration 8 nnz_H + 56 n, per FP64 residual 8 nnz_H + 52 n, with K and R
-    as executed; the compulsory bytes count one of each."""
+    as executed; the compulsory bytes count one of each. An island solved by
+    its (complex) FP64 factor as in arap_bytes."""
     K = st["cg_iters"].astype(np.float64)
     R = st["refinements"].astype(np.float64)
     nnz_h = 2.0 * nnz + 4.0 * nbnd
     cg = 8.0 * nnz_h + 56.0 * n
     rf = 8.0 * nnz_h + 52.0 * n
-    return float((K * cg + R * rf).sum()), float((cg + rf).sum())
+    factor = 4096.0 * blocks
+    return float((K * cg + R * rf + factor * (2.0 + 2.0 * R)).sum()), float((cg + rf).sum())
 
 
 class PlainBatch:
@@ -942,11 +955,13 @@ def main():
     arap_ms = float(np.mean([e[1].elapsed_time(e[2]) for e in ev]))
     lscm_ms = float(np.mean([e[0].elapsed_time(e[1]) for e in ev]))
     st = db.island_status()
+    blocks = factor_blocks(db)
     our_uvs = b.chart_uvs()
     db.setup(); db.lscm()                 # the LSCM solve's own counters
     st_lscm = db.island_status()
+    blocks_lscm = factor_blocks(db)
     n, t, nnz = _island_stats(b)
-    full, comp = arap_bytes(n, t, nnz, st)
+    full, comp = arap_bytes(n, t, nnz, st, blocks)
     units = float(tris * args.iters)
     if ws > 1:
         from ultimate_uv_artist_b200 import shard
@@ -984,14 +999,15 @@ def main():
             e2e_val = units_all / float(x[0])
 
     # our kernels per step: setup (k_frames, k_wpin, k_vert_isl, k_rows,
-    # k_far_pair, then k_coarse for the whole-CTA classes and for the rest),
-    # then k_islands for LSCM and for ARAP, each with k_wide before it when
-    # the batch has islands of the whole-GPU class
+    # k_far_pair, k_band, then k_coarse for the whole-CTA classes and for the
+    # rest), then k_direct, k_coarse (what the set-up left out and CG needs) and
+    # k_islands for LSCM and for ARAP, with k_wide before k_islands when the
+    # batch has islands of the whole-GPU class
     co = [int(db.desc.class_ofs[c]) for c in range(5)]
     big = min(max(co[2], 0), db.nc)
     n_coarse = int(big > 0) + int(db.nc - big > 0)
     n_wide = 2 if co[1] > co[0] else 0
-    launches_per_step = 5 + n_coarse + 2 + n_wide
+    launches_per_step = 6 + 3 * n_coarse + 2 + 1 + int(args.iters >= 3) + n_wide
     peaks = {}
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as fh:
@@ -1002,7 +1018,7 @@ def main():
     achieved = full / (arap_ms / 1e3) / 1e9
     achieved_c = comp / (arap_ms / 1e3) / 1e9
     nbnd = np.diff(db.plan.bofs.astype(np.int64))
-    lfull, lcomp = lscm_bytes(n, nnz, nbnd, st_lscm)
+    lfull, lcomp = lscm_bytes(n, nnz, nbnd, st_lscm, blocks_lscm)
 
     # the single-GPU legs (diagnostics beside the headline step) run only
     # without torchrun: a scaling run holds every GPU while rank 0 works
@@ -1093,18 +1109,18 @@ def main():
                        "l2": "inputs larger than L2 (about 1 GB resident per GPU)",
                        "step": "device frames+Laplacian, batched LSCM, 20 ARAP iterations",
                        "schedule": tuned},
-            "roofline": {"kernel": "k_islands<OP_ARAP>", "bound": "hbm", "achieved": achieved, "peak": hbm,
+            "roofline": {"kernel": "k_direct<OP_ARAP>", "bound": "hbm", "achieved": achieved, "peak": hbm,
                          "unit": "GB/s", "frac": achieved / hbm, "peak_source": peak_src,
-                         # DRAM read + write of one full-size ARAP launch, measured by
-                         # an ncu capture of this workload (summary under profiles/)
-                         "traffic": TRAFFIC_ARAP if args.islands == ISLANDS else None, "kernel_ms": arap_ms, "algorithmic_bytes": full,
+                         "note": "factors, right-hand sides and residuals streamed once per use; the "
+                                 "launch is bound by the largest island's chain of block steps",
+                         "traffic": None, "kernel_ms": arap_ms, "algorithmic_bytes": full,
+                         "direct_islands": int((blocks > 0).sum()),
                          "compulsory_bytes": comp, "compulsory_frac": achieved_c / hbm,
                          "cg_iters_total": int(st["cg_iters"].sum()),
                          "refinements_total": int(st["refinements"].sum()),
                          "max_resid": float(st["resid"].max())},
-            "roofline_lscm": {"kernel": "k_islands<OP_LSCM>", "bound": "hbm",
-                              "note": "streaming PCG model; the islands' vectors stay in shared memory and the "
-                                      "matrices in L2, so the model's bytes can exceed what HBM delivers",
+            "roofline_lscm": {"kernel": "k_direct<OP_LSCM>", "bound": "hbm",
+                              "note": "as roofline; the factors of the islands in flight stay in L2",
                               "achieved": lfull / (lscm_ms / 1e3) / 1e9, "peak": hbm, "unit": "GB/s",
                               "frac": lfull / (lscm_ms / 1e3) / 1e9 / hbm, "peak_source": peak_src,
                               "traffic": None, "kernel_ms": lscm_ms, "algorithmic_bytes": lfull,

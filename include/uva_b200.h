@@ -267,14 +267,19 @@ typedef struct uva_solve_params {
                                  takes the full step (engine/hier.py:549-552)   */
 } uva_solve_params;
 
-/* Frames, weights, matrix values, Jacobi diagonal, pins and pin weights.
+/* Frames, weights, matrix values, Jacobi diagonal, pins and pin weights; with
+ * b->band the elimination orders, and the coarse operators of CG only for
+ * islands without a factor (a solve builds the others when it needs them).
  * Batch semantics: global wpin = max|w| (gpu.py:138); param: per island.   */
 int uva_batch_setup(uva_batch* b, void* stream);
 /* LSCM of every island (hard pins at the far boundary pair, param.py:136-169)
- * solved by FP32 PCG with FP64 residual refinement; writes b->U.           */
+ * solved by an FP64 factor of each island (with b->direct) or by FP32 PCG
+ * with FP64 residual refinement; writes b->U.                              */
 int uva_lscm(uva_batch* b, const uva_solve_params* prm, void* stream);
 /* ARAP local/global iterations of every island in one persistent launch
- * (gpu.py:230-249 with semantics BATCH, param.py:379-414 with PARAM).      */
+ * (gpu.py:230-249 with semantics BATCH, param.py:379-414 with PARAM); with
+ * b->direct and at least 3 iterations, islands of up to 16,384 vertices by one
+ * FP64 factor each, in a launch before it.                                 */
 int uva_arap(uva_batch* b, const uva_solve_params* prm, void* stream);
 
 /* Step graphs. No counterpart in the reference, which launches every kernel
