@@ -482,8 +482,11 @@ def direct_parts(nv, slots):
     breadth-first order; the part holds 1.45 sqrt(n) and two blocks of 16
     (at most 16 blocks), a ring of 256 blocks, and the solve's vectors. An
     island whose factor needs more keeps the CG path."""
-    n = np.sort(np.asarray(nv, np.int64))[::-1][:slots].astype(np.float64)
-    n = np.where(n > _lib.DIRECT_MAX_N, 0, n)
+    n = np.sort(np.asarray(nv, np.int64))[::-1].astype(np.float64)
+    rest = n[slots:]
+    rest = rest[rest <= _lib.DIRECT_MAX_N]
+    # a CTA whose first island is too large for a factor still takes later ones
+    n = np.where(n > _lib.DIRECT_MAX_N, rest[0] if len(rest) else 0, n)[:slots]
     nblk = np.ceil(n / 16)
     blocks = nblk * np.minimum(np.ceil(1.45 * np.sqrt(n) / 16 + 2), 16) + 256
     ofs = np.zeros((2, slots + 1), np.int64)
