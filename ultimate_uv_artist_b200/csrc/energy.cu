@@ -94,8 +94,8 @@ __device__ __forceinline__ bool en_f(const EnTri& t, int kind, double& f, double
 
 // The forward pass gives a warp 32 * items consecutive triangles, lane by
 // lane. A lane sums its triangles of the same island (island ids do not
-// decrease along the triangles), then the warp folds lanes of equal islands,
-// so an island takes one FP64 atomic per warp. 5.1M triangles: 132 -> 82 us
+// decrease along the triangles), then the warp folds runs of lanes with equal
+// islands, so an island takes one FP64 atomic per run. 5.1M triangles: 132 -> 82 us
 // (a thread's own run of eight strided its loads by 128 bytes).
 __global__ void k_energy_fwd(const uva_batch b, const double* P, const double* U, int kind, int items, double* e_isl,
                              double* e_tri) {
@@ -123,16 +123,20 @@ __global__ void k_energy_fwd(const uva_batch b, const double* P, const double* U
         }
         acc += e;
     }
-    // fold the lanes' last islands, which do not decrease along the lanes
-    // (idle lanes carry -1 and never match a live one)
+    // Fold the lanes' last islands over contiguous runs of equal ids. In the
+    // last warp of the triangles some lanes end a row of 32 before the others,
+    // so one island can hold two runs (A A B B A A): each takes its own atomic.
+    const int prev = __shfl_up_sync(0xffffffffu, isl, 1);
+    const bool head = lane == 0 || prev != isl;
+    const unsigned heads = __ballot_sync(0xffffffffu, head);
+    const unsigned above = lane == 31 ? 0u : heads & (0xfffffffeu << lane);
+    const int end = above ? __ffs(above) - 1 : 32;   // one past the run's last lane
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const double y = __shfl_down_sync(0xffffffffu, acc, o);
-        const int yi = __shfl_down_sync(0xffffffffu, isl, o);
-        if (lane + o < 32 && yi == isl) acc += y;
+        if (lane + o < end) acc += y;
     }
-    const int prev = __shfl_up_sync(0xffffffffu, isl, 1);
-    if (isl >= 0 && (lane == 0 || prev != isl) && acc != 0.0) atomicAdd(e_isl + isl, acc);
+    if (isl >= 0 && head && acc != 0.0) atomicAdd(e_isl + isl, acc);
 }
 
 // The global FP64 additions bound the backward pass: L2 takes some 230 G of
