@@ -22,11 +22,15 @@ using namespace uva;
 
 namespace {
 
-// FP64 issue bounds these kernels as much as memory: one reciprocal square
-// root each for |e1| and |n| replaces two square roots and five divisions.
+// The frame, J and the energy use rounded roots and divisions: reciprocal roots
+// and products in their place put 4 % on the gradients' error (against 80 bits,
+// 24 charts: 1.67e-15 for 1.60e-15 in U, 1.94e-15 for 1.85e-15 in P) and lose a
+// triangle whose squared normal overflows, as inf * rsqrt(inf) is not a number.
+// 5.1M triangles: forward 126 us with them, 139 so; the backward's products of
+// reciprocals (1 / x1, 1 / y2, 1 / |n|) cost nothing in either.
 struct EnTri {
-    double e1[3], e2[3], nh[3];     // edges, unit normal
-    double il, x2, y2, iy2, area;   // 1 / x1, the frame, 1 / y2
+    double e1[3], e2[3], n[3];
+    double l1, nn, il, x2, y2, area;
     double j00, j01, j10, j11;
     bool live;
 };
@@ -40,23 +44,19 @@ __device__ __forceinline__ EnTri en_tri(const double* P, const double* U, int v0
     for (int k = 0; k < 3; ++k) { t.e1[k] = p1[k] - p0[k]; t.e2[k] = p2[k] - p0[k]; }
     const double2* UU = reinterpret_cast<const double2*>(U);
     const double2 u0 = UU[v0 + tv.x], u1 = UU[v0 + tv.y], u2 = UU[v0 + tv.z];
-    const double n0 = t.e1[1] * t.e2[2] - t.e1[2] * t.e2[1];
-    const double n1 = t.e1[2] * t.e2[0] - t.e1[0] * t.e2[2];
-    const double n2 = t.e1[0] * t.e2[1] - t.e1[1] * t.e2[0];
-    const double l1sq = t.e1[0] * t.e1[0] + t.e1[1] * t.e1[1] + t.e1[2] * t.e1[2];
-    const double nsq = n0 * n0 + n1 * n1 + n2 * n2;
-    const double inn = rsqrt(nsq), nn = nsq * inn;
-    t.il = rsqrt(l1sq);
+    t.n[0] = t.e1[1] * t.e2[2] - t.e1[2] * t.e2[1];
+    t.n[1] = t.e1[2] * t.e2[0] - t.e1[0] * t.e2[2];
+    t.n[2] = t.e1[0] * t.e2[1] - t.e1[1] * t.e2[0];
+    t.l1 = sqrt(t.e1[0] * t.e1[0] + t.e1[1] * t.e1[1] + t.e1[2] * t.e1[2]);   // x1
+    t.nn = sqrt(t.n[0] * t.n[0] + t.n[1] * t.n[1] + t.n[2] * t.n[2]);
+    t.il = 1.0 / fmax(t.l1, 1e-300);
     t.x2 = (t.e1[0] * t.e2[0] + t.e1[1] * t.e2[1] + t.e1[2] * t.e2[2]) * t.il;
-    t.y2 = nn * t.il;   // e2 . (n/|n| x e1/|e1|) = |n| / |e1|
-    t.iy2 = l1sq * t.il * inn;
-    t.area = 0.5 * nn;
-    // x1 y2 = |n|; a zero normal or edge makes nn or il not a number
-    t.live = nn >= 1e-300 && t.il <= 1e300;
-    t.nh[0] = n0 * inn; t.nh[1] = n1 * inn; t.nh[2] = n2 * inn;
+    t.y2 = t.nn * t.il;   // e2 . (n/|n| x e1/|e1|) = |n| / |e1|
+    t.area = 0.5 * t.nn;
+    t.live = fabs(t.l1 * t.y2) >= 1e-300;
     if (t.live) {
-        t.j00 = (u1.x - u0.x) * t.il; t.j10 = (u1.y - u0.y) * t.il;
-        t.j01 = ((u2.x - u0.x) - t.j00 * t.x2) * t.iy2; t.j11 = ((u2.y - u0.y) - t.j10 * t.x2) * t.iy2;
+        t.j00 = (u1.x - u0.x) / t.l1; t.j10 = (u1.y - u0.y) / t.l1;
+        t.j01 = ((u2.x - u0.x) - t.j00 * t.x2) / t.y2; t.j11 = ((u2.y - u0.y) - t.j10 * t.x2) / t.y2;
     } else {
         t.j00 = t.j01 = t.j10 = t.j11 = 0.0;
     }
@@ -68,10 +68,10 @@ __device__ __forceinline__ bool en_f(const EnTri& t, int kind, double& f, double
     if (kind == 0) {
         const double qe = 0.5 * (t.j00 + t.j11), qh = 0.5 * (t.j10 - t.j01);
         const double rf = 0.5 * (t.j00 - t.j11), rg = 0.5 * (t.j10 + t.j01);
-        const double q2 = qe * qe + qh * qh;
-        const double iq = q2 > 0.0 ? rsqrt(q2) : 0.0, q = q2 * iq, r = sqrt(rf * rf + rg * rg);
+        const double q = sqrt(qe * qe + qh * qh), r = sqrt(rf * rf + rg * rg);
         f = (q + r - 1.0) * (q + r - 1.0) + (q - r - 1.0) * (q - r - 1.0);
-        const double c = qe * iq, s = qh * iq;
+        double c = 0.0, s = 0.0;
+        if (q > 0.0) { c = qe / q; s = qh / q; }
         G[0] = 2.0 * (t.j00 - c); G[1] = 2.0 * (t.j01 + s); G[2] = 2.0 * (t.j10 - s); G[3] = 2.0 * (t.j11 - c);
         return true;
     }
@@ -82,9 +82,9 @@ __device__ __forceinline__ bool en_f(const EnTri& t, int kind, double& f, double
         G[0] = G[1] = G[2] = G[3] = 0.0;
         return false;
     }
-    const double id = 1.0 / det, id2 = id * id;
+    const double id2 = 1.0 / (det * det);
     f = fro + fro * id2 - 4.0;
-    const double a = 2.0 * (1.0 + id2), b = -2.0 * fro * id2 * id;
+    const double a = 2.0 * (1.0 + id2), b = -2.0 * fro * id2 / det;
     G[0] = a * t.j00 + b * t.j11;
     G[1] = a * t.j01 - b * t.j10;
     G[2] = a * t.j10 - b * t.j01;
@@ -95,8 +95,8 @@ __device__ __forceinline__ bool en_f(const EnTri& t, int kind, double& f, double
 // The forward pass gives a warp 32 * items consecutive triangles, lane by
 // lane. A lane sums its triangles of the same island (island ids do not
 // decrease along the triangles), then the warp folds runs of lanes with equal
-// islands, so an island takes one FP64 atomic per run. 5.1M triangles: 132 -> 82 us
-// (a thread's own run of eight strided its loads by 128 bytes).
+// islands, so an island takes one FP64 atomic per run. 5.1M triangles: 166 -> 139 us
+// with its launches (a thread's own run of eight strided its loads by 128 bytes).
 __global__ void k_energy_fwd(const uva_batch b, const double* P, const double* U, int kind, int items, double* e_isl,
                              double* e_tri) {
     const int lane = threadIdx.x & 31;
@@ -144,8 +144,9 @@ __global__ void k_energy_fwd(const uva_batch b, const double* P, const double* U
 // The corner gradients therefore pass through shared memory, and the lanes of
 // an addition take the components of a vertex side by side: one or two
 // operations per corner instead of five. 512 islands of 5.1M triangles, UV and
-// position gradients: 316 -> 192 us. (Summing a block's corners by vertex in a
-// shared hash table first took 281 us: its lookups cost more than they save.)
+// position gradients, with their launches: 350 -> 243 us. (Summing a block's
+// corners by vertex in a shared hash table first took 281 us in place of 192
+// without them: its lookups cost more than they save.)
 constexpr int kBwdNT = 128;
 
 template <bool POS>
@@ -168,29 +169,29 @@ __global__ void __launch_bounds__(kBwdNT) k_energy_bwd(const uva_batch b, const 
             // dE/dJ = A G; J = D M^-1 with D = [du1 du2]: dE/dD = dE/dJ M^-T
             // M^-1 = [[1/x1, -x2/(x1 y2)], [0, 1/y2]]
             const double g00 = A * G[0], g01 = A * G[1], g10 = A * G[2], g11 = A * G[3];
-            const double m01 = -t.x2 * t.il * t.iy2;
-            const double d1x = g00 * t.il + g01 * m01, d2x = g01 * t.iy2;
-            const double d1y = g10 * t.il + g11 * m01, d2y = g11 * t.iy2;
+            const double il = t.il, iy2 = 1.0 / t.y2, m01 = -t.x2 * il * iy2;
+            const double d1x = g00 * il + g01 * m01, d2x = g01 * iy2;
+            const double d1y = g10 * il + g11 * m01, d2y = g11 * iy2;
             double* o = su[threadIdx.x];
             o[0] = -(d1x + d2x); o[1] = -(d1y + d2y);
             o[2] = d1x; o[3] = d1y;
             o[4] = d2x; o[5] = d2y;
             if constexpr (POS) {
-                // dE/dM = -J^T (A G) M^-T
+                // dE/dM = -J^T (A G) M^-T; M^-T = [[1/x1, 0], [m01, 1/y2]]
                 const double jg00 = t.j00 * g00 + t.j10 * g10, jg01 = t.j00 * g01 + t.j10 * g11;
                 const double jg11 = t.j01 * g01 + t.j11 * g11;
-                const double dM00 = -(jg00 * t.il + jg01 * m01);   // d/dx1
-                const double dM01 = -(jg01 * t.iy2);                // d/dx2 (row 0, col 1)
-                const double dM11 = -(jg11 * t.iy2);                // d/dy2
+                const double dM00 = -(jg00 * il + jg01 * m01);   // d/dx1
+                const double dM01 = -(jg01 * iy2);                // d/dx2 (row 0, col 1)
+                const double dM11 = -(jg11 * iy2);                // d/dy2
                 // x1 = |e1|, x2 = e1.e2 / |e1|, y2 = |n| / |e1|, area = |n| / 2;
                 // d|n|/de1 = e2 x nh, d|n|/de2 = nh x e1
-                const double il2 = t.il * t.il;
-                const double a1 = dM00 * t.il - il2 * (dM01 * t.x2 + dM11 * t.y2), a2 = dM01 * t.il;
-                const double an = dM11 * t.il + 0.5 * sc * f_;
-                const double dn1[3] = {t.e2[1] * t.nh[2] - t.e2[2] * t.nh[1], t.e2[2] * t.nh[0] - t.e2[0] * t.nh[2],
-                                       t.e2[0] * t.nh[1] - t.e2[1] * t.nh[0]};
-                const double dn2[3] = {t.nh[1] * t.e1[2] - t.nh[2] * t.e1[1], t.nh[2] * t.e1[0] - t.nh[0] * t.e1[2],
-                                       t.nh[0] * t.e1[1] - t.nh[1] * t.e1[0]};
+                const double inn = 1.0 / t.nn, il2 = il * il;
+                const double a1 = dM00 * il - il2 * (dM01 * t.x2 + dM11 * t.y2), a2 = dM01 * il;
+                const double an = (dM11 * il + 0.5 * sc * f_) * inn;
+                const double dn1[3] = {t.e2[1] * t.n[2] - t.e2[2] * t.n[1], t.e2[2] * t.n[0] - t.e2[0] * t.n[2],
+                                       t.e2[0] * t.n[1] - t.e2[1] * t.n[0]};
+                const double dn2[3] = {t.n[1] * t.e1[2] - t.n[2] * t.e1[1], t.n[2] * t.e1[0] - t.n[0] * t.e1[2],
+                                       t.n[0] * t.e1[1] - t.n[1] * t.e1[0]};
                 double* w = sp[threadIdx.x];
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
