@@ -55,6 +55,8 @@ extern "C" {
 #define UVA_ST_NOBOUNDARY 8   /* LSCM: no boundary loop                     */
 #define UVA_ST_BADCLASS   16  /* island above its team's capacity (class_ofs
                                   inconsistent with the sizes); not solved      */
+#define UVA_ST_TIMEOUT    32  /* a wait inside the direct solver ran out after
+                                  outer_iters iterations; U holds those         */
 
 typedef struct uva_island_status {
     int32_t cg_iters;      /* inner FP32 CG iterations executed             */

@@ -26,6 +26,7 @@ ST_NONFINITE = 2
 ST_ENERGYSTOP = 4
 ST_NOBOUNDARY = 8
 ST_BADCLASS = 16
+ST_TIMEOUT = 32
 
 PLAN_NSIZES = 9
 STEP_SETUP, STEP_LSCM, STEP_ARAP = 1, 2, 4

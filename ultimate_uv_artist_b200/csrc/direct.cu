@@ -56,6 +56,7 @@
 #include "common.cuh"
 #include "direct.cuh"
 #include "island.cuh"
+#include "wait.cuh"
 
 using namespace uva;
 
@@ -175,20 +176,21 @@ __device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, %0;" 
 __device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Bounded wait: false after about a second without the phase.
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
-    for (int it = 0; it < (1 << 18); ++it) {
-        unsigned ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
+constexpr int kWaitPolls = 1 << 18;      // about a second without the phase
+__device__ __forceinline__ bool mbar_wait(int& bad, unsigned bar, unsigned parity) {
+    return bounded_wait(
+        [=]() {
+            unsigned ok;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok)
+                : "r"(bar), "r"(parity)
+                : "memory");
+            return ok != 0;
+        },
+        kWaitPolls, bad);
 }
 __device__ __forceinline__ void bulk_copy(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -531,7 +533,11 @@ __device__ void factor(const Isl& I, Shared& S, double* stage) {
 // right-hand side of its current row stays in registers until the row is
 // final, then the group publishes it and takes the row 16 further on. The
 // last warp feeds the ring: it copies a step's blocks once the compute warps
-// have released the stage.
+// have released the stage. A wait that runs out sets S.bad: the feeding warp
+// stops copying, the compute warps go through their steps without waiting (on
+// whatever the stages hold), and the feeding warp waits for the copies in
+// flight. rb is then worthless, which the caller's FP64 residual shows: a
+// solution that misses the tolerance with S.bad set is not used.
 template <Op OP>
 __device__ void solve(Isl& I, Shared& S, double* stage) {
     constexpr bool CP = OP == OP_LSCM;
@@ -546,11 +552,13 @@ __device__ void solve(Isl& I, Shared& S, double* stage) {
         if (++q == NS) { q = 0; ph ^= 1; }
     };
     if (tid >= kCT) {
-        for (int K = 0; K < nblk; ++K) {   // column K's blocks, one copy each
+        bool run = true;
+        for (int K = 0; K < nblk && run; ++K) {   // column K's blocks, one copy each
             const int R = K + 1 + lane;
             const bool on = lane < kMaxW && R < nblk && S.first[min(R, kMaxBlk)] <= K;
             const unsigned cnt = __popc(__ballot_sync(0xffffffffu, on));
-            if (!mbar_wait(empty0 + 8 * q, ph ^ 1)) S.bad = 2;
+            run = __all_sync(0xffffffffu, mbar_wait(S.bad, empty0 + 8 * q, ph ^ 1));
+            if (!run) break;
             if (lane == 0) mbar_expect(full0 + 8 * q, cnt * kBytes);
             __syncwarp();
             if (on)
@@ -558,9 +566,10 @@ __device__ void solve(Isl& I, Shared& S, double* stage) {
                           I.L + static_cast<size_t>(S.off[R] + K - S.first[R]) * BB, kBytes, full0 + 8 * q);
             next();
         }
-        for (int K = nblk - 1; K >= 0; --K) {   // row K's blocks are contiguous
+        for (int K = nblk - 1; K >= 0 && run; --K) {   // row K's blocks are contiguous
             const unsigned bytes = (K - S.first[K]) * kBytes;
-            if (!mbar_wait(empty0 + 8 * q, ph ^ 1)) S.bad = 2;
+            run = __all_sync(0xffffffffu, mbar_wait(S.bad, empty0 + 8 * q, ph ^ 1));
+            if (!run) break;
             if (lane == 0) {
                 mbar_expect(full0 + 8 * q, bytes);
                 if (bytes)
@@ -585,7 +594,7 @@ __device__ void solve(Isl& I, Shared& S, double* stage) {
                 if (R + 16 < nblk) nxt = I.rb[(R + 16) * kNB + r];
             }
             compute_sync();   // r_K visible
-            if (!mbar_wait(full0 + 8 * q, ph)) S.bad = 2;
+            mbar_wait(S.bad, full0 + 8 * q, ph);
             if (fr <= K) {
                 const double* B = stage + q * stage_d + (R - K - 1) * BB;
                 const double2* x = S.xk[K & 1];
@@ -643,7 +652,7 @@ __device__ void solve(Isl& I, Shared& S, double* stage) {
             }
             const int f = S.first[K];
             compute_sync();
-            if (!mbar_wait(full0 + 8 * q, ph)) S.bad = 2;
+            mbar_wait(S.bad, full0 + 8 * q, ph);
             if (J >= f) {   // J < K
                 const double* B = stage + q * stage_d + (J - f) * BB;
                 const double2* x = S.xk[K & 1];
@@ -671,11 +680,23 @@ __device__ void solve(Isl& I, Shared& S, double* stage) {
     I.q = q;
     I.ph = ph;
     __syncthreads();
+    if (S.bad) {   // uniform: the copies in flight land before the stages are used for anything else
+        if (tid >= kCT) {
+            int late = 0;
+            for (int k = 0; k < NS; ++k) {   // (a stage never copied into counts as there)
+                if (--q < 0) { q = NS - 1; ph ^= 1; }
+                mbar_wait(late, full0 + 8 * q, ph);
+            }
+        }
+        __syncthreads();
+    }
 }
 
 // ------------------------------------------------------------------ ARAP
 // gpu.py:230-249 / param.py:379-414. False (with U untouched) when the first
-// global step does not reach the tolerance: the CG path takes the island.
+// global step does not reach the tolerance or a wait ran out in it: the CG path
+// takes the island. A wait that runs out later leaves U as the iterations
+// before it made it, with UVA_ST_TIMEOUT.
 __device__ bool solve_arap(const uva_batch& b, const uva_solve_params& prm, Isl& I, Shared& S, Red& rd, double* stage) {
     const int tid = threadIdx.x;
     const bool batch = b.semantics == UVA_SEM_BATCH;
@@ -757,7 +778,7 @@ __device__ bool solve_arap(const uva_batch& b, const uva_solve_params& prm, Isl&
             // an ill-conditioned island gets one more solve even within the tolerance
             const double few = ref == 0 ? 1e-11 / fmax(prm.tol, 1e-11) : 1.0;
             if (rr[0] <= t0 * few * few && rr[1] <= t1 * few * few) break;
-            if (ref >= min(prm.max_refine, 3) || !isfinite(rr[0] + rr[1])) {
+            if (ref >= min(prm.max_refine, 3) || !isfinite(rr[0] + rr[1]) || S.bad) {
                 capped = !(rr[0] <= t0 && rr[1] <= t1);
                 break;
             }
@@ -765,7 +786,11 @@ __device__ bool solve_arap(const uva_batch& b, const uva_solve_params& prm, Isl&
             __syncthreads();
         }
         if (capped) {
-            if (it == 0 && !bad) return false;
+            if (it == 0 && (!bad || S.bad)) return false;
+            if (S.bad) {
+                st.flags |= UVA_ST_TIMEOUT;
+                break;
+            }
             st.flags |= UVA_ST_MAXITER;
         }
         st.outer_iters = it + 1;
@@ -808,7 +833,7 @@ __device__ bool solve_arap(const uva_batch& b, const uva_solve_params& prm, Isl&
 
 // ------------------------------------------------------------------ LSCM
 // Hard pins p0 -> (0,0), p1 -> (|P[p1]-P[p0]|, 0), param.py:136-169. False
-// when the residual stays above the tolerance.
+// when the residual stays above the tolerance or a wait ran out.
 __device__ bool solve_lscm(const uva_batch& b, const uva_solve_params& prm, Isl& I, Shared& S, Red& rd, double* stage) {
     const int tid = threadIdx.x;
     double2* x64 = reinterpret_cast<double2*>(b.x64) + I.v0;
@@ -845,7 +870,7 @@ __device__ bool solve_lscm(const uva_batch& b, const uva_solve_params& prm, Isl&
         // an ill-conditioned island (a long strip) gets one more solve even
         // within the tolerance
         const bool good = rr[0] <= 1e-22 * fmax(bb, 1e-300);
-        if ((done && (good || ref > 1)) || ref > min(prm.max_refine, 3) || !isfinite(rr[0])) break;
+        if ((done && (good || ref > 1)) || ref > min(prm.max_refine, 3) || !isfinite(rr[0]) || (ref > 0 && S.bad)) break;
         solve<OP_LSCM>(I, S, stage);
         for (int i = tid; i < I.n; i += kNT) {
             const double2 d = I.rb[__ldg(I.pos + i)];
@@ -877,6 +902,7 @@ __global__ void __launch_bounds__(kNT, 2) k_direct(uva_batch b, uva_solve_params
     const int64_t room = ofs[blockIdx.x + 1] - ofs[blockIdx.x];
     Red rd{S.red, 0};
     int rank = blockIdx.x;
+    bool dead = false;   // a wait ran out: the CTA leaves its further islands to CG
     while (rank < b.nc) {
         Isl I;
         I.id = b.order[rank];
@@ -892,7 +918,7 @@ __global__ void __launch_bounds__(kNT, 2) k_direct(uva_batch b, uva_solve_params
         const int64_t need = (static_cast<int64_t>(total) + 256) * BB * 8 + static_cast<int64_t>(npad) * 16 * (CP ? 1 : 3);
         bool done = false;
         const long long t0 = global_ns();
-        if ((info[0] & 1) && need <= room) {
+        if (!dead && (info[0] & 1) && need <= room) {
             const int32_t* first = band_first(b, I.v0, I.id);
             I.pin = b.vert_row[I.v0 + b.pins[3 * I.id]];
             const int q0 = b.pins[3 * I.id + 1], q1 = b.pins[3 * I.id + 2];
@@ -956,7 +982,7 @@ __global__ void __launch_bounds__(kNT, 2) k_direct(uva_batch b, uva_solve_params
                 if (S.bad == 0) {
                     if (CP) done = solve_lscm(b, prm, I, S, rd, stage);
                     else done = solve_arap(b, prm, I, S, rd, stage);
-                    if (S.bad) done = false;
+                    dead = S.bad == 2;
                 }
             }
             __syncthreads();
