@@ -207,11 +207,15 @@ typedef struct uva_batch {
                                  FP16 scaled to a largest entry of 1024, then
                                  the inverse scale (FP32)                      */
     float*  coarse_l;         /* 4*cofs[nc] floats: the same for LSCM          */
-    double* coarse_work;      /* 4*cofs[nc]: FP64 workspace of the setup        */
+    double* coarse_work;      /* 4*cofs[nc]: FP64 workspace of the setup, and of
+                                 uva_lscm / uva_arap / uva_batch_coarse, so not
+                                 the caller's between them. Null in a solve: no
+                                 whole-GPU team, and Jacobi for the islands whose
+                                 operators the set-up left out (see band)      */
     float*  cpart;            /* 2*nslices floats of solve scratch: the whole-GPU
                                  team of islands above 16,384 vertices keeps its
                                  grid barrier here (and its reduction slots in
-                                 coarse_work, free after the setup)           */
+                                 coarse_work)                                 */
     int32_t class_ofs[5];     /* host values: class c owns order[ofs[c]..ofs[c+1]) */
     /* geometry, written by uva_batch_setup */
     const double*  P;         /* n*3 positions (FP64)                          */
@@ -238,7 +242,12 @@ typedef struct uva_batch {
                                  null: 2 updates kept in p32/d32/q32/r32        */
     /* direct solver of islands up to 16,384 vertices (all optional; null: CG) */
     int32_t* band;            /* n + n/16 + 5*nc ints: elimination order, skyline
-                                 and state per island, written by the setup     */
+                                 and state per island, written by the setup and
+                                 by uva_lscm / uva_arap (state). With it the
+                                 set-up leaves out the coarse operators of islands
+                                 that a factor can solve, and the first uva_lscm /
+                                 uva_arap that gives one to CG writes them to
+                                 coarse_a and coarse_l                          */
     unsigned char* direct;    /* factor scratch of uva_lscm / uva_arap           */
     const int64_t* direct_ofs;/* device, 2*(direct_slots+1): byte offsets of the
                                  CTAs' parts, for ARAP then for LSCM: part j is
@@ -274,6 +283,10 @@ typedef struct uva_solve_params {
  * islands without a factor (a solve builds the others when it needs them).
  * Batch semantics: global wpin = max|w| (gpu.py:138); param: per island.   */
 int uva_batch_setup(uva_batch* b, void* stream);
+/* The coarse operators that the set-up left out (b->band), for every island:
+ * once before calls of uva_arap_noalloc. Nothing to do without band, or when a
+ * solve has built them.                                                     */
+int uva_batch_coarse(uva_batch* b, void* stream);
 /* LSCM of every island (hard pins at the far boundary pair, param.py:136-169)
  * solved by an FP64 factor of each island (with b->direct) or by FP32 PCG
  * with FP64 residual refinement; writes b->U.                              */
@@ -319,7 +332,9 @@ int uva_slim(uva_batch* b, const uva_solve_params* prm, double* scratch, void* s
  * (x64, b64, rc, r32, d32, p32, q32, cpart, work, hist) is ignored and replaced by one
  * static device array of 7,602,432 bytes that every GPU loading the library
  * holds until exit. The caller still passes the inputs (topology, geometry,
- * pins, order) and the outputs (U, status). Limits: at most 32768 vertices
+ * pins, order, coarse operators) and the outputs (U, status). With band, islands
+ * whose coarse operators are not built take CG with Jacobi, to the same
+ * tolerance in more iterations: call uva_batch_coarse once after the set-up. Limits: at most 32768 vertices
  * and 65536 triangles per call, else UVA_E_TOOBIG. The first call on a device
  * looks up the array's device address (cudaGetSymbolAddress); make that first
  * call before any stream capture. All calls share the array and it keeps the

@@ -98,6 +98,7 @@ _SIGS = {
     "uva_batch_setup": [vp, vp],
     "uva_lscm": [vp, vp, vp],
     "uva_arap": [vp, vp, vp],
+    "uva_batch_coarse": [vp, vp],
     "uva_arap_noalloc": [vp, vp, vp],
     "uva_slim": [vp, vp, vp, vp],
     "uva_slim_scratch_bytes": [vp, vp],

@@ -530,6 +530,7 @@ __device__ __forceinline__ Isl load_island(const uva_batch& b, int isl) {
     I.p0 = p0 >= 0 ? b.vert_row[I.v0 + p0] : -1;
     I.p1 = p1 >= 0 ? b.vert_row[I.v0 + p1] : -1;
     I.agg = b.agg_rows[isl];
+    if (b.band && !(band_info(b, isl)[0] & 2)) I.agg = 0;   // coarse operators not built: Jacobi only
     I.M = I.agg > 0 ? (I.n + I.agg - 1) / I.agg : 0;
     I.co = b.cofs[isl];
     I.aggsh = (I.agg > 0 && (I.agg & (I.agg - 1)) == 0) ? __ffs(I.agg) - 1 : -1;
@@ -1775,7 +1776,10 @@ constexpr size_t kCoarseSmallSmem = sizeof(double2) * kCoarseSmallM * kCoarseSma
 // launches this again with `left` set, for the islands it is about to give to
 // CG without one (ARAP calls of few iterations, no scratch, a zero pivot):
 // 1.8 ms of the set-up of 2,000 islands, 0.31 of one of 6,100 triangles;
-// the launch that finds nothing to do takes 2 us (one island) to 7.
+// the launch that finds nothing to do takes 2 us (one island) to 7. Bit 1 of
+// an island's info[0] says that its operators are built; CG goes without them
+// (Jacobi) where it is not set: no coarse_work, or uva_arap_noalloc, which
+// writes none of the caller's arrays, without uva_batch_coarse before it.
 template <int NT>
 __global__ void __launch_bounds__(NT) k_coarse(uva_batch b, int first, int count, int left) {
     extern __shared__ __align__(16) double wsm[];
@@ -1967,7 +1971,7 @@ constexpr int kDirectMinIters = 3;
 bool direct_ready(const uva_batch* b) { return b->band && b->direct && b->direct_ofs && b->direct_slots > 0; }
 
 template <Op OP>
-int launch_islands(const uva_batch* b, const uva_solve_params* prm, cudaStream_t s) {
+int launch_islands(const uva_batch* b, const uva_solve_params* prm, cudaStream_t s, bool build_coarse = true) {
     if (!check_classes(b)) {
         uva_set_error("uva_arap/uva_lscm: class_ofs must be 0 <= ... <= nc, non-decreasing");
         return UVA_E_ARG;
@@ -1980,7 +1984,7 @@ int launch_islands(const uva_batch* b, const uva_solve_params* prm, cudaStream_t
         const int rc = uva_direct_launch(b, prm, OP == OP_LSCM, s);
         if (rc != UVA_OK) return rc;
     }
-    if (b->band) {   // coarse operators that the set-up left out and these islands need
+    if (b->band && build_coarse) {   // coarse operators that the set-up left out and these islands need
         e = launch_coarse(b, true, s);
         if (e != cudaSuccess) return uva_cuda_status(e, "uva_islands/coarse");
     }
@@ -2325,6 +2329,19 @@ extern "C" int uva_batch_setup(uva_batch* b, void* stream) {
     return UVA_OK;
 }
 
+extern "C" int uva_batch_coarse(uva_batch* b, void* stream) {
+    if (!check_batch_inputs(b) || (b->nc > 0 && b->band && !b->coarse_work)) {
+        uva_set_error("uva_batch_coarse: bad arguments (coarse_work is required)");
+        return UVA_E_ARG;
+    }
+    if (b->nc == 0 || !b->band) return UVA_OK;   // no elimination order: the set-up built them all
+    uva_batch w = *b;
+    w.direct = nullptr;   // every island's, whatever the last solve did
+    const cudaError_t e = launch_coarse(&w, true, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return uva_cuda_status(e, "uva_batch_coarse");
+    return UVA_OK;
+}
+
 extern "C" int uva_arap(uva_batch* b, const uva_solve_params* prm, void* stream) {
     if (!check_batch(b) || !prm) { uva_set_error("uva_arap: bad arguments"); return UVA_E_ARG; }
     if (b->nc == 0 || prm->iters <= 0) return UVA_OK;
@@ -2491,7 +2508,7 @@ extern "C" int uva_arap_noalloc(const uva_batch* b, const uva_solve_params* prm,
     const int rc = noalloc_scratch(&base);
     if (rc != UVA_OK) return rc;
     uva_batch w = *b;
-    w.direct = nullptr;   // the caller's scratch too
+    w.direct = nullptr;   // the caller's scratch too; coarse operators only as they are (const batch)
     size_t off = 0;
     w.work = reinterpret_cast<int32_t*>(base + off); off += kNaWork;
     w.x64 = reinterpret_cast<double*>(base + off); off += kNaX64;
@@ -2505,5 +2522,5 @@ extern "C" int uva_arap_noalloc(const uva_batch* b, const uva_solve_params* prm,
     w.hist = reinterpret_cast<float*>(base + off);
     // the work counters are the only scratch that must start at zero;
     // launch_islands clears them on the stream before the launch
-    return launch_islands<OP_ARAP>(&w, prm, static_cast<cudaStream_t>(stream));
+    return launch_islands<OP_ARAP>(&w, prm, static_cast<cudaStream_t>(stream), false);
 }
