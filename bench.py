@@ -1000,14 +1000,15 @@ def main():
 
     # our kernels per step: setup (k_frames, k_wpin, k_vert_isl, k_rows,
     # k_far_pair, k_band, then k_coarse for the whole-CTA classes and for the
-    # rest), then k_direct, k_coarse (what the set-up left out and CG needs) and
-    # k_islands for LSCM and for ARAP, with k_wide before k_islands when the
+    # rest), then k_choose (not for a few small islands), k_direct, k_coarse (what
+    # the set-up left out and CG needs) and k_islands for LSCM and for ARAP, with k_wide before k_islands when the
     # batch has islands of the whole-GPU class
     co = [int(db.desc.class_ofs[c]) for c in range(5)]
     big = min(max(co[2], 0), db.nc)
     n_coarse = int(big > 0) + int(db.nc - big > 0)
     n_wide = 2 if co[1] > co[0] else 0
-    launches_per_step = 6 + 3 * n_coarse + 2 + 1 + int(args.iters >= 3) + n_wide
+    n_direct = (1 + int(db.desc.maxrows > 700 or db.nc > 592)) * (1 + int(args.iters >= 3))
+    launches_per_step = 6 + 3 * n_coarse + 2 + n_direct + n_wide
     peaks = {}
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as fh:

@@ -32,6 +32,7 @@ PLAN_NSIZES = 9
 STEP_SETUP, STEP_LSCM, STEP_ARAP = 1, 2, 4
 CLASS_BIG, CLASS_MID, CLASS_SMALL = 8192, 2048, 256
 DIRECT_MAX_N = 16384   # islands above keep the CG path (direct.cuh)
+DIRECT_MIN_ITERS = 3   # ARAP calls of fewer iterations keep it too (solve.cu)
 (PLAN_NC, PLAN_N, PLAN_T, PLAN_E, PLAN_NSLICES, PLAN_NSLOTS, PLAN_NBVERTS, PLAN_MAXROWS, PLAN_NCOARSE) = range(9)
 
 vp = C.c_void_p

@@ -46,7 +46,8 @@
 // An island keeps the CG path (solve.cu, launched after this kernel) when it
 // is above kDirectMaxN vertices, not connected, wider than kMaxW blocks, when
 // its factor does not fit the CTA's scratch, or when a pivot or the residual
-// check says that its operator is singular.
+// check says that its operator is singular; all islands of a launch do when
+// k_choose expects CG to be faster.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -887,6 +888,119 @@ __device__ bool solve_lscm(const uva_batch& b, const uva_solve_params& prm, Isl&
     return true;
 }
 
+// Bytes of an island's factor, ring of G and vectors.
+template <Op OP>
+__device__ __forceinline__ int64_t factor_bytes(int blocks, int nblk) {
+    constexpr bool CP = OP == OP_LSCM;
+    return (static_cast<int64_t>(blocks) + 256) * kBE * (CP ? 2 : 1) * 8 + static_cast<int64_t>(nblk) * kNB * 16 * (CP ? 1 : 3);
+}
+
+// ------------------------------------------------------------------ choice
+// Factors or CG for a launch: estimates of both in microseconds, from the
+// island sizes. Measured on disks of 32 to 16,000 vertices, 1 to 20,000 of
+// them, alike and uneven, 3 to 20 ARAP iterations, at the default tolerances
+// (70 batches): the estimates are within 15 % for factors, 30 % for CG, whose
+// iterations depend on the shape.
+//  * Factors: a chain of block columns and of substitutions per island,
+//    proportional to its vertices (`lat`), two CTAs per SM; slower by up to a
+//    third once the launch's factors exceed the L2.
+//  * CG: a warp, a quarter CTA or a CTA per island by size class (up to 256,
+//    2,048, 8,192 vertices, above: vectors in global memory), an SM's time per
+//    vertex (`thr`) when there are more islands than teams.
+// ARAP has the factors' chain in every iteration, so few islands of 5,000 to
+// 8,000 vertices are faster by CG, whose CTA has 1,024 threads for them: 20
+// iterations of 400 uneven islands (20 to 7,904 vertices) 24.3 ms by factors,
+// 16.7 by CG; of one island of 8,061: 19.0 and 15.6; but of 2,000 uneven ones
+// 29.9 and 39.4, of 1,200 islands of 877 12.5 and 19.0. LSCM is slower by
+// factors only for thousands of islands of some 60 vertices and fewer: 20,000
+// of 24: 1.58 ms and 0.69.
+// Islands without a factor take CG after the others: where one of them lasts as
+// long as the launch by CG alone would, the factors' launch before it is time
+// lost (60 irregular charts of 3,000 vertices, 10 with a factor: ARAP 19.9 ms, 11.9
+// by CG alone).
+struct Cost {
+    float lat, thr;
+};
+template <Op OP>
+__device__ __forceinline__ Cost factor_cost(float n, float iters) {
+    const float t = OP == OP_ARAP ? 15.f + 3.f * iters + n * (0.33f + 1.9e-5f * n + 0.093f * iters)
+                                  : 8.f + n * (0.53f + 4.5e-5f * n);
+    return {t, t * fminf(1.55f, 1.15f + 2e-4f * n)};
+}
+template <Op OP>
+__device__ __forceinline__ Cost cg_cost(float n, float iters) {
+    if (OP == OP_ARAP) {
+        const float k = sqrtf(iters);   // later iterations start near their solution
+        return {n <= UVA_CLASS_SMALL ? 9.f * k * n
+                                     : (n <= UVA_CLASS_MID ? 0.95f * k * n : (n <= UVA_CLASS_BIG ? 1.f : 3.f) * k * (1300.f + 0.28f * n)),
+                n <= 128.f ? n * (0.3f * iters - 0.3f) : 0.42f * k * n};
+    }
+    return {n * (n <= UVA_CLASS_SMALL ? 6.f : (n <= UVA_CLASS_BIG ? 3.2f : 8.6f)),
+            n * (n <= 400.f ? 0.12f + 0.0032f * n : (n <= UVA_CLASS_MID ? 1.4f : 4.f))};
+}
+
+// work[kWorkCg] = 1: CG for the whole launch. Islands above kDirectMaxN have
+// their own launch either way and are left out.
+template <Op OP>
+__global__ void __launch_bounds__(1024) k_choose(uva_batch b, uva_solve_params prm) {
+    __shared__ float part[32][7];
+    const int64_t* ofs = b.direct_ofs + (OP == OP_LSCM ? b.direct_slots + 1 : 0);
+    const float iters = static_cast<float>(prm.iters);
+    // 0 longest factor, 1 sum of factors, 2 their vertices, 3 longest of the
+    // CG islands, 4 their sum, 5 longest of all by CG, 6 their sum
+    float v[7] = {};
+    for (int r = threadIdx.x; r < b.nc; r += 1024) {
+        const int isl = b.order[r], n = b.vofs[isl + 1] - b.vofs[isl];
+        if (n > kDirectMaxN) continue;
+        const int32_t* info = band_info(b, isl);
+        const int part_of = min(r, b.direct_slots - 1);
+        const bool takes = (info[0] & 1) &&
+                           factor_bytes<OP>(info[1], (n + kNB - 1) / kNB) <= ofs[part_of + 1] - ofs[part_of];
+        const Cost cg = cg_cost<OP>(static_cast<float>(n), iters);
+        v[5] = fmaxf(v[5], cg.lat);
+        v[6] += cg.thr;
+        if (takes) {
+            const Cost f = factor_cost<OP>(static_cast<float>(n), iters);
+            v[0] = fmaxf(v[0], f.lat);
+            v[1] += f.thr;
+            v[2] += static_cast<float>(n);
+        } else {
+            v[3] = fmaxf(v[3], cg.lat);
+            v[4] += cg.thr;
+        }
+    }
+    constexpr unsigned kMax = 1u | 8u | 32u;   // 0, 3, 5: maxima, the others sums
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float y = __shfl_xor_sync(0xffffffffu, v[k], o);
+            v[k] = kMax >> k & 1 ? fmaxf(v[k], y) : v[k] + y;
+        }
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][k] = v[k];
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 32; ++w)
+#pragma unroll
+        for (int k = 0; k < 7; ++k) v[k] = kMax >> k & 1 ? fmaxf(v[k], part[w][k]) : v[k] + part[w][k];
+    constexpr float kSMs = 148.f;
+    // a tighter tolerance takes CG more iterations
+    const float tight = logf(fmaxf(static_cast<float>(prm.tol), 1e-30f)) / logf(OP == OP_ARAP ? 2e-7f : 1e-8f);
+    auto both = [&](float lat, float sum) { return tight * sqrtf(lat * lat + sum * sum / (kSMs * kSMs)); };
+    const float spill = fminf(1.f, v[2] / 4e5f);
+    // CTAs beside one another: the launch's, or two per SM where each has one island
+    const float ctas = b.direct_slots < b.nc ? static_cast<float>(b.direct_slots) : 2.f * kSMs;
+    const float direct = fmaxf(v[0] * (1.f + (OP == OP_ARAP ? 0.35f : 0.2f) * spill), v[1] / ctas);
+    // charts without a factor are irregular ones, on which CG took some 1.5
+    // times the iterations that it takes on disks; an estimate so rough counts
+    // from half a millisecond
+    const float shape = v[3] > 0.f ? 1.5f : 1.f;
+    const float rest = shape * both(v[3], v[4]), all = shape * both(v[5], v[6]);
+    const float gain = direct + rest - all;
+    if (v[2] > 0.f && gain > 0.05f * (direct + rest) && (rest == 0.f || gain > 500.f)) b.work[kWorkCg] = 1;
+}
+
 // One CTA per island, largest first; CTA j starts with the j-th island (its
 // scratch is sized for that one, the later ones are smaller). info[3] of an
 // island tells the CG launch that follows whether it is done.
@@ -897,6 +1011,11 @@ __global__ void __launch_bounds__(kNT, 2) k_direct(uva_batch b, uva_solve_params
     extern __shared__ __align__(128) double stage[];
     __shared__ Shared S;
     const int tid = threadIdx.x;
+    if (b.work[kWorkCg]) {
+        for (int r = blockIdx.x * kNT + tid; r < b.nc; r += gridDim.x * kNT) band_info(b, b.order[r])[3] = 0;
+        if (blockIdx.x == 0 && tid == 0) b.work[kWorkLeft] = b.nc;
+        return;
+    }
     const int64_t* ofs = b.direct_ofs + (CP ? b.direct_slots + 1 : 0);
     unsigned char* mem = b.direct + ofs[blockIdx.x];
     const int64_t room = ofs[blockIdx.x + 1] - ofs[blockIdx.x];
@@ -915,7 +1034,7 @@ __global__ void __launch_bounds__(kNT, 2) k_direct(uva_batch b, uva_solve_params
         int32_t* info = band_info(b, I.id);
         const int total = info[1];
         const int npad = I.nblk * kNB;
-        const int64_t need = (static_cast<int64_t>(total) + 256) * BB * 8 + static_cast<int64_t>(npad) * 16 * (CP ? 1 : 3);
+        const int64_t need = factor_bytes<OP>(total, I.nblk);
         bool done = false;
         const long long t0 = global_ns();
         if (!dead && (info[0] & 1) && need <= room) {
@@ -1047,6 +1166,13 @@ int uva_direct_launch(const uva_batch* b, const uva_solve_params* prm, bool lscm
     const cudaError_t e = lscm ? direct_attr<OP_LSCM>() : direct_attr<OP_ARAP>();
     if (e != cudaSuccess) return uva_cuda_status(e, "uva_direct/cudaFuncSetAttribute");
     const int grid = std::min(b->nc, b->direct_slots);
+    // few and small islands: factors won every measurement, and even irregular
+    // charts of up to 700 vertices fit (the choice would cost 4 of some 120 us)
+    if (b->maxrows > 700 || b->nc > 592) {
+        if (lscm) k_choose<OP_LSCM><<<1, 1024, 0, s>>>(*b, *prm);
+        else k_choose<OP_ARAP><<<1, 1024, 0, s>>>(*b, *prm);
+        UVA_CHECK_LAUNCH("uva_direct/choose");
+    }
     if (lscm) k_direct<OP_LSCM><<<grid, kNT, kRing, s>>>(*b, *prm);
     else k_direct<OP_ARAP><<<grid, kNT, kRing, s>>>(*b, *prm);
     UVA_CHECK_LAUNCH(lscm ? "uva_lscm/direct" : "uva_arap/direct");

@@ -7,7 +7,7 @@
 
 constexpr int kDirectMaxN = 16384;   // vertices of an island (band positions fit 14 bits)
 // counters in uva_batch.work beside the CG path's four
-constexpr int kWorkNext = 4, kWorkLeft = 5;
+constexpr int kWorkNext = 4, kWorkLeft = 5, kWorkCg = 6;
 
 // uva_batch.band: position of every solver row (n), first block column of
 // every block row (n / 16 + nc), then 4 ints per island: a factor is possible

@@ -663,7 +663,7 @@ class DeviceBatch:
     def arap(self, iters=8, line_search=True, energy_tol=0.0, **kw):
         kw.setdefault("rev_ctas", self.rev_ctas)
         prm = self.params("arap", iters=iters, line_search=line_search, energy_tol=energy_tol, **kw)
-        D, scratch = self._with_direct("arap") if prm.iters > 0 else (self.desc, None)
+        D, scratch = self._with_direct("arap") if prm.iters >= _lib.DIRECT_MIN_ITERS else (self.desc, None)
         check(_lib.lib().uva_arap(C.byref(D), C.byref(prm), self._stream()), "uva_arap")
 
     def slim(self, iters=10, energy_tol=1e-5, cg_tol=1e-13, cg_max=50000):
@@ -794,7 +794,7 @@ class StepGraph:
         self._lp = db.params("lscm", **lscm_kw)
         self._ap = db.params("arap", iters=max(arap_iters, 1), line_search=line_search, **arap_kw)
         h = C.c_void_p()
-        kinds = (["lscm"] if lscm else []) + (["arap"] if arap_iters > 0 else [])
+        kinds = (["lscm"] if lscm else []) + (["arap"] if arap_iters >= _lib.DIRECT_MIN_ITERS else [])
         D, self._scratch = db._with_direct(*kinds) if kinds else (db.desc, None)
         check(_lib.lib().uva_step_graph_create(C.byref(D), parts, C.byref(self._lp), C.byref(self._ap),
                                                C.byref(h)), "uva_step_graph_create")
