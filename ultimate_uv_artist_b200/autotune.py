@@ -6,12 +6,13 @@ sub-team instead of one warp (``small``), and how many CTAs start with the
 small-island classes (``rev_ctas``, which keeps long-lived small islands out
 of the launch's tail). The best choice depends on the batch's island-size
 distribution and on the device, so ``tune`` times short ARAP and LSCM runs
-of the batch itself under each candidate (CUDA events, UVs restored after
-every trial) and applies the fastest. Results are cached per device and
+of the batch itself by CG alone under each candidate (CUDA events, UVs restored
+after every trial) and applies the fastest. Results are cached per device and
 size signature; ``tune`` is meant for a warm-up, not for a timed region.
 """
 from __future__ import annotations
 
+import ctypes as C
 import itertools
 
 import numpy as np
@@ -60,6 +61,12 @@ def _time(fn, dev):
     return e0.elapsed_time(e1)
 
 
+def _cg(db, kind, **kw):
+    """One LSCM or ARAP call without scratch for factors: every island by CG."""
+    prm = db.params(kind, **kw)
+    _lib.check(getattr(_lib.lib(), "uva_" + kind)(C.byref(db.desc), C.byref(prm), db._stream()), "uva_" + kind)
+
+
 def tune(db, arap_iters=3, candidates=None, use_cache=True):
     """Choose (mid, small, rev_ctas) for DeviceBatch ``db``; returns the
     chosen setting and the measured milliseconds of every candidate."""
@@ -71,11 +78,13 @@ def tune(db, arap_iters=3, candidates=None, use_cache=True):
         db.rev_ctas = best["rev_ctas"]
         return best, {}
     U0 = db.U.clone()
+    # the coarse operators that the set-up left out, outside the trials
+    _lib.check(_lib.lib().uva_batch_coarse(C.byref(db.desc), db._stream()), "uva_batch_coarse")
     results = {}
     for mid, small, rev in itertools.product(cand["mid"], cand["small"], cand["rev_ctas"]):
         db.set_classes(mid, small)
-        ms = _time(lambda: db.lscm(rev_ctas=rev), db.dev)
-        ms += _time(lambda: db.arap(iters=arap_iters, rev_ctas=rev), db.dev)
+        ms = _time(lambda: _cg(db, "lscm", rev_ctas=rev), db.dev)
+        ms += _time(lambda: _cg(db, "arap", iters=arap_iters, rev_ctas=rev), db.dev)
         results[(mid, small, rev)] = ms
         db.U.copy_(U0)
     (mid, small, rev), _ = min(results.items(), key=lambda kv: kv[1])
