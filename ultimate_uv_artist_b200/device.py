@@ -18,6 +18,7 @@ from __future__ import annotations
 import contextlib
 import ctypes as C
 import threading
+import warnings
 
 import numpy as np
 import torch
@@ -616,7 +617,8 @@ class DeviceBatch:
     def _with_direct(self, *kinds):
         """(descriptor, scratch): the batch's descriptor with factor scratch
         for the calls of ``kinds``, from torch's caching allocator on the
-        batch's stream; without memory for it the descriptor as it is (CG)."""
+        batch's stream; without memory for it the descriptor as it is (CG),
+        with a RuntimeWarning."""
         nbytes = max(int(self._direct_parts[0 if k == "arap" else 1][-1]) for k in kinds)
         if nbytes == 0:
             return self.desc, None
@@ -624,6 +626,8 @@ class DeviceBatch:
             with (torch.cuda.stream(self.stream) if self.stream is not None else contextlib.nullcontext()):
                 scratch = torch.empty(nbytes, dtype=torch.uint8, device=self.dev)
         except torch.cuda.OutOfMemoryError:
+            warnings.warn(f"no device memory for the factors of {' and '.join(kinds)} ({nbytes / 1e9:.1f} GB): conjugate "
+                          "gradients, to the call's tolerance but slower", RuntimeWarning, stacklevel=3)
             return self.desc, None
         D = _lib.BatchDesc.from_buffer_copy(self.desc)
         D.direct = scratch.data_ptr()
