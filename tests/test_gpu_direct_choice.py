@@ -49,7 +49,8 @@ def _same(U, V, vofs):
 CASES = {
     "one_small": ([(20, 20)], 20, True, True),
     "one_large_few_iterations": ([(88, 90)], 3, True, True),
-    "one_large": ([(88, 90)], 20, True, False),                       # the factor's chain, iteration after iteration
+    "one_large": ([(88, 90)], 20, True, True),                        # too near to call: factors
+    "some_large": ([(88, 90)] * 60 + [(40, 40)] * 100, 20, True, False),   # the factors' chains, out of L2
     "above_the_cta_class": ([(100, 100)], 20, True, True),            # CG's vectors would be in global memory
     "many_mid": ([(30, 30)] * 700, 8, True, True),
     "large_among_many": ([(88, 90)] * 8 + [(30, 30)] * 3000, 20, True, True),   # the others fill the launch
@@ -73,7 +74,8 @@ def test_choice_and_results(cuda, name):
     db.arap(iters=iters)
     st = db.island_status()
     assert ((st["cg_iters"] == 0) == arap_f).all()
-    assert (st["flags"] == 0).all() and (st["resid"] <= 2e-7 * 1.001).all() and (st["outer_iters"] == iters).all()
+    assert (st["flags"] == 0).all() and (st["outer_iters"] == iters).all()
+    assert (st["resid"] <= 1e-7 * 1.001).all()      # in place of a factor CG takes half the tolerance
     U_a = db.uvs().copy()
     db.U[:db.n].copy_(start)
     g = db.step_graph(setup=False, lscm=False, arap_iters=iters)     # the same choice in a captured call

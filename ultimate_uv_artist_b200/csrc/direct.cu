@@ -910,14 +910,14 @@ __device__ __forceinline__ int64_t factor_bytes(int blocks, int nblk) {
 // ARAP has the factors' chain in every iteration, so few islands of 5,000 to
 // 8,000 vertices are faster by CG, whose CTA has 1,024 threads for them: 20
 // iterations of 400 uneven islands (20 to 7,904 vertices) 24.3 ms by factors,
-// 16.7 by CG; of one island of 8,061: 19.0 and 15.6; but of 2,000 uneven ones
+// 16.7 by CG; of 100 of them 20.6 and 13.2; but of 2,000 uneven ones
 // 29.9 and 39.4, of 1,200 islands of 877 12.5 and 19.0. LSCM is slower by
 // factors only for thousands of islands of some 60 vertices and fewer: 20,000
 // of 24: 1.58 ms and 0.69.
 // Islands without a factor take CG after the others: where one of them lasts as
 // long as the launch by CG alone would, the factors' launch before it is time
 // lost (60 irregular charts of 3,000 vertices, 10 with a factor: ARAP 19.9 ms, 11.9
-// by CG alone).
+// by CG alone). CG is taken when it is expected to save an eighth.
 struct Cost {
     float lat, thr;
 };
@@ -980,25 +980,33 @@ __global__ void __launch_bounds__(1024) k_choose(uva_batch b, uva_solve_params p
         if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][k] = v[k];
     }
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    for (int w = 1; w < 32; ++w)
 #pragma unroll
-        for (int k = 0; k < 7; ++k) v[k] = kMax >> k & 1 ? fmaxf(v[k], part[w][k]) : v[k] + part[w][k];
+    for (int k = 0; k < 7; ++k) {   // on every thread
+        v[k] = part[0][k];
+        for (int w = 1; w < 32; ++w) v[k] = kMax >> k & 1 ? fmaxf(v[k], part[w][k]) : v[k] + part[w][k];
+    }
     constexpr float kSMs = 148.f;
-    // a tighter tolerance takes CG more iterations
-    const float tight = logf(fmaxf(static_cast<float>(prm.tol), 1e-30f)) / logf(OP == OP_ARAP ? 2e-7f : 1e-8f);
+    // a tighter tolerance takes CG more iterations; ARAP islands that could have
+    // a factor are solved to half of it (solve.cu), an eighth more time
+    const float tight = (OP == OP_ARAP ? 1.12f : 1.f) *
+                        logf(fmaxf(static_cast<float>(prm.tol), 1e-30f)) / logf(OP == OP_ARAP ? 2e-7f : 1e-8f);
     auto both = [&](float lat, float sum) { return tight * sqrtf(lat * lat + sum * sum / (kSMs * kSMs)); };
     const float spill = fminf(1.f, v[2] / 4e5f);
     // CTAs beside one another: the launch's, or two per SM where each has one island
     const float ctas = b.direct_slots < b.nc ? static_cast<float>(b.direct_slots) : 2.f * kSMs;
     const float direct = fmaxf(v[0] * (1.f + (OP == OP_ARAP ? 0.35f : 0.2f) * spill), v[1] / ctas);
-    // charts without a factor are irregular ones, on which CG took some 1.5
-    // times the iterations that it takes on disks; an estimate so rough counts
-    // from half a millisecond
-    const float shape = v[3] > 0.f ? 1.5f : 1.f;
+    // charts without a factor are irregular ones, on which CG takes longer than on
+    // disks (ARAP some 1.5 times, LSCM 1.15); so rough an estimate counts from
+    // half a millisecond
+    const float shape = v[3] > 0.f ? (OP == OP_ARAP ? 1.5f : 1.15f) : 1.f;
     const float rest = shape * both(v[3], v[4]), all = shape * both(v[5], v[6]);
     const float gain = direct + rest - all;
-    if (v[2] > 0.f && gain > 0.05f * (direct + rest) && (rest == 0.f || gain > 500.f)) b.work[kWorkCg] = 1;
+    if (!(v[2] > 0.f && gain > 0.12f * (direct + rest) && (rest == 0.f || gain > 500.f))) return;
+    for (int r = threadIdx.x; r < b.nc; r += 1024) band_info(b, r)[3] = 0;
+    if (threadIdx.x == 0) {
+        b.work[kWorkLeft] = b.nc;
+        b.work[kWorkCg] = 1;
+    }
 }
 
 // One CTA per island, largest first; CTA j starts with the j-th island (its
@@ -1011,11 +1019,7 @@ __global__ void __launch_bounds__(kNT, 2) k_direct(uva_batch b, uva_solve_params
     extern __shared__ __align__(128) double stage[];
     __shared__ Shared S;
     const int tid = threadIdx.x;
-    if (b.work[kWorkCg]) {
-        for (int r = blockIdx.x * kNT + tid; r < b.nc; r += gridDim.x * kNT) band_info(b, b.order[r])[3] = 0;
-        if (blockIdx.x == 0 && tid == 0) b.work[kWorkLeft] = b.nc;
-        return;
-    }
+    if (b.work[kWorkCg]) return;   // every island is left
     const int64_t* ofs = b.direct_ofs + (CP ? b.direct_slots + 1 : 0);
     unsigned char* mem = b.direct + ofs[blockIdx.x];
     const int64_t room = ofs[blockIdx.x + 1] - ofs[blockIdx.x];
