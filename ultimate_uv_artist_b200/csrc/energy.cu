@@ -22,12 +22,49 @@ using namespace uva;
 
 namespace {
 
-// The frame, J and the energy use rounded roots and divisions: reciprocal roots
-// and products in their place put 4 % on the gradients' error (against 80 bits,
-// 24 charts: 1.67e-15 for 1.60e-15 in U, 1.94e-15 for 1.85e-15 in P) and lose a
-// triangle whose squared normal overflows, as inf * rsqrt(inf) is not a number.
-// 5.1M triangles: forward 126 us with them, 139 so; the backward's products of
-// reciprocals (1 / x1, 1 / y2, 1 / |n|) cost nothing in either.
+// Value of one triangle's energy, for the forward pass, by reciprocal square
+// roots and products: FP64 issue bounds that pass as much as memory (5.1M
+// triangles: 124 us with its launches, 139 with rounded roots and divisions), and
+// the rounding of an island's sum covers theirs (24 charts, against 80 bits: 2e-16
+// to 3e-16 either way). inf * rsqrt(inf) is not a number, so a squared normal that
+// overflows counts as an infinite one.
+__device__ __forceinline__ double en_value(const double* P, const double* U, int v0, int4 tv, int kind) {
+    const double* p0 = P + 3 * (v0 + tv.x);
+    const double* p1 = P + 3 * (v0 + tv.y);
+    const double* p2 = P + 3 * (v0 + tv.z);
+    double e1[3], e2[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { e1[k] = p1[k] - p0[k]; e2[k] = p2[k] - p0[k]; }
+    const double2* UU = reinterpret_cast<const double2*>(U);
+    const double2 u0 = UU[v0 + tv.x], u1 = UU[v0 + tv.y], u2 = UU[v0 + tv.z];
+    const double n0 = e1[1] * e2[2] - e1[2] * e2[1], n1 = e1[2] * e2[0] - e1[0] * e2[2], n2 = e1[0] * e2[1] - e1[1] * e2[0];
+    const double l1sq = e1[0] * e1[0] + e1[1] * e1[1] + e1[2] * e1[2];
+    const double nsq = n0 * n0 + n1 * n1 + n2 * n2;
+    const double inn = rsqrt(nsq), nn = isinf(nsq) ? nsq : nsq * inn, il = rsqrt(l1sq);
+    // x1 y2 = |n|; a zero normal or edge makes nn or il not a number, and a
+    // first edge beyond 1e154 has no frame
+    if (!(nn >= 1e-300 && il <= 1e300 && il > 0.0)) return 0.0;
+    const double x2 = (e1[0] * e2[0] + e1[1] * e2[1] + e1[2] * e2[2]) * il;
+    const double iy2 = l1sq * il * inn;   // y2 = e2 . (n/|n| x e1/|e1|) = |n| / |e1|
+    const double j00 = (u1.x - u0.x) * il, j10 = (u1.y - u0.y) * il;
+    const double j01 = ((u2.x - u0.x) - j00 * x2) * iy2, j11 = ((u2.y - u0.y) - j10 * x2) * iy2;
+    const double area = 0.5 * nn;
+    if (kind == 0) {
+        const double qe = 0.5 * (j00 + j11), qh = 0.5 * (j10 - j01), rf = 0.5 * (j00 - j11), rg = 0.5 * (j10 + j01);
+        const double q = sqrt(qe * qe + qh * qh), r = sqrt(rf * rf + rg * rg);
+        return area * ((q + r - 1.0) * (q + r - 1.0) + (q - r - 1.0) * (q - r - 1.0));
+    }
+    const double det = j00 * j11 - j01 * j10;
+    if (!(det > 0.0)) return area * INFINITY;
+    const double fro = j00 * j00 + j01 * j01 + j10 * j10 + j11 * j11;
+    return area * (fro + fro / (det * det) - 4.0);
+}
+
+// The backward pass: rounded roots and divisions in the frame, J and the
+// energy's terms, which reciprocal roots in their place would put 4 % on the
+// gradients' error (24 charts, against 80 bits: 1.67e-15 for 1.60e-15 in U,
+// 1.94e-15 for 1.85e-15 in P); products of three reciprocals (1 / x1, 1 / y2,
+// 1 / |n|) after that, which add nothing to it.
 struct EnTri {
     double e1[3], e2[3], n[3];
     double l1, nn, il, x2, y2, area;
@@ -95,7 +132,7 @@ __device__ __forceinline__ bool en_f(const EnTri& t, int kind, double& f, double
 // The forward pass gives a warp 32 * items consecutive triangles, lane by
 // lane. A lane sums its triangles of the same island (island ids do not
 // decrease along the triangles), then the warp folds runs of lanes with equal
-// islands, so an island takes one FP64 atomic per run. 5.1M triangles: 166 -> 139 us
+// islands, so an island takes one FP64 atomic per run. 5.1M triangles: 166 -> 124 us
 // with its launches (a thread's own run of eight strided its loads by 128 bytes).
 __global__ void k_energy_fwd(const uva_batch b, const double* P, const double* U, int kind, int items, double* e_isl,
                              double* e_tri) {
@@ -108,13 +145,7 @@ __global__ void k_energy_fwd(const uva_batch b, const double* P, const double* U
         const int64_t f = f0 + 32 * k;
         if (f >= b.t) break;
         const int4 tv = reinterpret_cast<const int4*>(b.tri4)[f];
-        const EnTri t = en_tri(P, U, b.vofs[tv.w], tv);
-        double e = 0.0;
-        if (t.live) {
-            double f_, G[4];
-            en_f(t, kind, f_, G);
-            e = t.area * f_;
-        }
+        const double e = en_value(P, U, b.vofs[tv.w], tv, kind);
         if (e_tri) e_tri[f] = e;
         if (tv.w != isl) {   // a new island: flush the previous one
             if (isl >= 0 && acc != 0.0) atomicAdd(e_isl + isl, acc);
