@@ -1110,17 +1110,18 @@ def main():
                        "l2": "inputs larger than L2 (about 1 GB resident per GPU)",
                        "step": "device frames+Laplacian, batched LSCM, 20 ARAP iterations",
                        "schedule": tuned},
-            "roofline": {"kernel": "k_direct<OP_ARAP>", "bound": "hbm", "achieved": achieved, "peak": hbm,
+            "roofline": {"kernel": "k_direct<OP_ARAP>", "bound": "latency", "achieved": achieved, "peak": hbm,
                          "unit": "GB/s", "frac": achieved / hbm, "peak_source": peak_src,
-                         "note": "factors, right-hand sides and residuals streamed once per use; the "
-                                 "launch is bound by the largest island's chain of block steps",
+                         "note": "model bytes: factors, right-hand sides and residuals streamed once per use "
+                                 "against the copy rate; the launch is bound by the largest island's chain "
+                                 "of block steps",
                          "traffic": None, "kernel_ms": arap_ms, "algorithmic_bytes": full,
                          "direct_islands": int((blocks > 0).sum()),
                          "compulsory_bytes": comp, "compulsory_frac": achieved_c / hbm,
                          "cg_iters_total": int(st["cg_iters"].sum()),
                          "refinements_total": int(st["refinements"].sum()),
                          "max_resid": float(st["resid"].max())},
-            "roofline_lscm": {"kernel": "k_direct<OP_LSCM>", "bound": "hbm",
+            "roofline_lscm": {"kernel": "k_direct<OP_LSCM>", "bound": "latency",
                               "note": "as roofline; the factors of the islands in flight stay in L2",
                               "achieved": lfull / (lscm_ms / 1e3) / 1e9, "peak": hbm, "unit": "GB/s",
                               "frac": lfull / (lscm_ms / 1e3) / 1e9 / hbm, "peak_source": peak_src,

@@ -288,13 +288,15 @@ int uva_batch_setup(uva_batch* b, void* stream);
  * solve has built them.                                                     */
 int uva_batch_coarse(uva_batch* b, void* stream);
 /* LSCM of every island (hard pins at the far boundary pair, param.py:136-169)
- * solved by an FP64 factor of each island (with b->direct) or by FP32 PCG
- * with FP64 residual refinement; writes b->U.                              */
+ * solved by an FP64 factor of each island (with b->direct, unless PCG is
+ * expected to be faster for the batch's sizes) or by FP32 PCG with FP64
+ * residual refinement; writes b->U.                                        */
 int uva_lscm(uva_batch* b, const uva_solve_params* prm, void* stream);
 /* ARAP local/global iterations of every island in one persistent launch
  * (gpu.py:230-249 with semantics BATCH, param.py:379-414 with PARAM); with
  * b->direct and at least 3 iterations, islands of up to 16,384 vertices by one
- * FP64 factor each, in a launch before it.                                 */
+ * FP64 factor each, in a launch before it, unless PCG is expected to be faster
+ * for the batch's sizes: such islands are then solved to half of prm->tol.  */
 int uva_arap(uva_batch* b, const uva_solve_params* prm, void* stream);
 
 /* Step graphs. No counterpart in the reference, which launches every kernel

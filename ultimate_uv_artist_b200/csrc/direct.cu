@@ -2,14 +2,14 @@
 // in FP64, one CTA per island, in place of the conjugate gradients of
 // solve.cu for islands of up to kDirectMaxN vertices.
 //
-// Why: a chart is a planar graph, so in breadth-first order its matrix has a
-// narrow skyline (about the square root of n). An 8,061-vertex disk has
-// 3,779 blocks of 16 x 16 in its factor: 27 million multiply-adds and 7.7 MB,
-// where the FP32 two-level CG needs 1,416 iterations of LSCM (and some 40
-// per ARAP step) whose cost is barriers and L2 round trips. The factor is
-// exact to FP64 round-off, so one solve per global step meets the tolerance
-// that the FP64 residual check asks for; ARAP factors once per call and
-// only substitutes in its iterations.
+// Why: in breadth-first order the matrix of a chart has a narrow skyline (about
+// the square root of n columns on a regular grid, up to twice that on irregular
+// triangulations). An 8,061-vertex disk has 3,779 blocks of 16 x 16 in its
+// factor: 27 million multiply-adds and 7.7 MB, where the FP32 two-level CG needs
+// 1,416 iterations of LSCM (and some 40 per ARAP step) whose cost is barriers and
+// L2 round trips. The factor is exact to FP64 round-off, so one solve per global
+// step meets the tolerance that the FP64 residual check asks for; ARAP factors
+// once per call and only substitutes in its iterations.
 //
 //   k_band    (set-up) Cuthill-McKee order of an island from its far boundary
 //             vertex: level-synchronous breadth-first search, levels ordered
@@ -33,11 +33,12 @@
 // islands (8,061 vertices the largest). Its substitutions are a chain of 504
 // steps of 960 cycles, three fifths of them shared-memory loads and the FP64
 // sums, the rest the hand-over of the block and its barrier: 11.7 ms of the
-// 29.9 ms ARAP launch of 20 iterations; local step, right-hand side, residual
-// and line search take 11.4, the factor 4.5. With CG: 40.0 ms LSCM, 39.6 ARAP.
+// 29.1 ms ARAP launch of 20 iterations; local step, right-hand side, residual
+// and line search take 11.4, the factor some 4. With CG: 40.0 ms LSCM, 39.6 ARAP.
 // Tried and slower: fragments of L prefetched in registers from global memory
 // (45 ms ARAP), block x vector on the tensor instruction (36), the same layout
-// with scalar sums and two feeding warps (29.9 ARAP, but 12.7 LSCM).
+// with scalar sums and two feeding warps (29.9 ARAP, 29.9 then without them, but
+// 12.7 LSCM).
 //
 // Blocks are stored column by column with an XOR swizzle (element (r, c) at
 // 16 c + (r ^ c)): a forward step reads a column over 16 lanes, a backward
@@ -921,7 +922,7 @@ __device__ __forceinline__ int64_t factor_bytes(int blocks, int nblk) {
 // 8,000 vertices are faster by CG, whose CTA has 1,024 threads for them: 20
 // iterations of 400 uneven islands (20 to 7,904 vertices) 24.3 ms by factors,
 // 16.7 by CG; of 100 of them 20.6 and 13.2; but of 2,000 uneven ones
-// 29.9 and 39.4, of 1,200 islands of 877 12.5 and 19.0. LSCM is slower by
+// 29.1 and 39.4, of 1,200 islands of 877 12.5 and 19.0. LSCM is slower by
 // factors only for thousands of islands of some 60 vertices and fewer: 20,000
 // of 24: 1.58 ms and 0.69.
 // Islands without a factor take CG after the others: where one of them lasts as

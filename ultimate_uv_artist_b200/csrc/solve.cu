@@ -14,9 +14,9 @@
 //    near-singular soft-pinned system well posed in FP32.
 //  * Islands of up to 16,384 vertices are solved by FP64 factors (direct.cu,
 //    launched first); what follows holds for the others: larger or wide ones,
-//    those whose factor does not fit its scratch or has a zero pivot, ARAP
-//    calls of fewer than kDirectMinIters iterations, and callers without the
-//    factor's scratch.
+//    those whose factor does not fit its scratch or has a zero pivot, launches
+//    on which CG is expected to be faster, ARAP calls of fewer than
+//    kDirectMinIters iterations, and callers without the factor's scratch.
 //  * Mixed precision: each global step solves L x = b with FP32 Jacobi-PCG
 //    corrections and recomputes the residual b - L x in FP64 (iterative
 //    refinement) until ||b - L x|| <= tol ||b|| per column, checked in FP64.

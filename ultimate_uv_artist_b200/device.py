@@ -31,7 +31,8 @@ from ._lib import check, ptr
 # UV extent) from exact solves on 2,000 uneven islands; at 2e-7 they stay
 # below 4e-6, for about 13 % more CG iterations (islands of up to 16,384
 # vertices are solved by FP64 factors, to some 1e-13, and only checked against
-# it; figures here are those of the CG path). Inner FP32 solves aim at a
+# it, or to half of it where CG is faster; figures here are those of the CG
+# path). Inner FP32 solves aim at a
 # 1e-5 reduction (or the final tolerance): fewer FP64 restarts than 1e-3.
 # LSCM solves to 1e-8: on the same islands (12 size-stratified ones against
 # the FP64 oracle) the LSCM UVs stay within 4.5e-7 of exact solves and the
@@ -479,10 +480,11 @@ def direct_parts(nv, slots):
     """Byte offsets (2, slots + 1) of the direct solver's scratch, ARAP then
     LSCM: one part per CTA, sized for the CTA's first island (islands of
     ``nv`` vertices are taken largest first, so the later ones are smaller).
-    A planar chart's factor has about 0.95 sqrt(n) columns per row in
-    breadth-first order; the part holds 1.45 sqrt(n) and two blocks of 16
-    (at most 16 blocks), a ring of 256 blocks, and the solve's vectors. An
-    island whose factor needs more keeps the CG path."""
+    The factor of a disk cut from a regular grid has about 0.95 sqrt(n) columns
+    per row in breadth-first order; the part holds 1.45 sqrt(n) and two blocks of
+    16 (at most 16 blocks), a ring of 256 blocks, and the solve's vectors. An
+    island whose factor needs more keeps the CG path, as most irregular
+    triangulations above some 2,000 vertices do."""
     n = np.sort(np.asarray(nv, np.int64))[::-1].astype(np.float64)
     rest = n[slots:]
     rest = rest[rest <= _lib.DIRECT_MAX_N]

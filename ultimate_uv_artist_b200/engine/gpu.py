@@ -9,8 +9,8 @@ Same public surface as the reference module (engine/gpu.py:16-299):
 What changes underneath: every Batch computation runs in the uva_b200 CUDA
 kernels (sm_100a) on a device-resident batch. A global step is solved per
 island to ||b - L x|| <= 2e-7 ||b|| per column, checked in FP64 (FP64 factors for
-islands of up to 16,384 vertices, FP32 CG with FP64 residual refinement for the
-others), instead of at most 40 CG iterations with a 1e-6
+islands of up to 16,384 vertices, FP32 CG with FP64 residual refinement where no
+factor fits or CG is faster), instead of at most 40 CG iterations with a 1e-6
 stop test on the whole batch and a host sync per iteration. UVs are kept in FP64 on the device;
 ``U`` returns them in the Batch dtype. There is no CPU path: constructing a
 Batch without a CUDA device raises RuntimeError.
